@@ -131,7 +131,7 @@ int Engine::layout()
     nmax_ = 16;
     maxb_ = 0;
     int tag_base = 0, coeff_off = 0, mass_off = 0, bond_off = 0, rdf_off = 0;
-    any_mdpd_ = any_dpd_ = bonds_ = rdf_ = any_gc_ = false;
+    any_mdpd_ = any_dpd_ = bonds_ = rdf_ = any_gc_ = filt_ = false;
     for (size_t r = 0; r < reps_.size(); r++) {
         Replica& R = reps_[r];
         RepDesc& d = R.desc;
@@ -177,6 +177,7 @@ int Engine::layout()
         d.rcmax2 = (float)(rcm * rcm);
         const float hs = (float)(R.in.skin * 0.5);
         d.hskin2 = hs * hs;
+        if (d.cut2 > d.rcmax2) filt_ = true;
         d.skin_zero = R.in.skin == 0.0;
         d.ntypes = R.sys.n_atomtypes;
         d.coeff_off = coeff_off;
@@ -348,8 +349,8 @@ int Engine::alloc_and_upload()
                 const double A = c[0], B = c[1], gamma = c[2], rc = c[3], rd = c[4];
                 const size_t o = d.coeff_off + (size_t)(ti * nt + tj) * 3;
                 const float rcf = (float)rc;
-                coeff[o] = make_float4((float)A, (float)gamma, (float)(std::sqrt(gamma) * sig_scale), rcf * rcf);
-                coeff[o + 1] = make_float4((float)(1.0 / rc), (float)(0.5 * A * rc), (float)B,
+                coeff[o] = make_float4((float)A, (float)gamma, (float)(std::sqrt(gamma) * sig_scale), (float)(1.0 / rc));
+                coeff[o + 1] = make_float4(rcf * rcf, (float)(0.5 * A * rc), (float)B,
                                            rd > 0 ? (float)(1.0 / rd) : 0.0f);
                 const float rdf = (float)rd;
                 coeff[o + 2] = make_float4(rdf * rdf, (float)(0.25 * B * rd),
@@ -740,10 +741,10 @@ static StepArgs step_args(const DeviceBuffers& b, int P, int nmax, int maxb, int
 // launch overlaps the tail of its predecessor (every step kernel starts with
 // griddep_wait(), which orders it after the predecessor's memory).
 template <typename... KArgs, typename... Args>
-static void pdl_launch(void (*kern)(KArgs...), int grid, int block, cudaStream_t s, Args... args)
+static void pdl_launch(void (*kern)(KArgs...), dim3 grid, int block, cudaStream_t s, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)block);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
@@ -773,24 +774,33 @@ static void pdl_launch_smem(void (*kern)(KArgs...), int grid, int block, size_t 
     cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// the flattened schedules (4..9): one launch for any step (split = false) or two
+template <int STYLE, bool BONDS, bool FILT>
+static void launch_flat(bool split, cudaStream_t s, const StepArgs& a)
+{
+    const int threads = DPD_FLAT_WARPS * 32, grid = (a.P + threads - 1) / threads;
+    if (!split) {
+        // several warps per 32 particles while the GPU has room for them: 24000 particles
+        // take 21.7 / 16.3 / 14.3 / 14.4 us with 1 / 2 / 4 / 8 parts, 81000 25.4 / 25.1 / 26.4
+        // with 1 / 2 / 4, 192000 44.2 / 44.3 / 50.0
+        const int warps = a.P / 32;
+        const int parts = warps <= 148 * 6 ? 4 : (warps <= 148 * 20 ? 2 : 1);
+        pdl_launch(k_pair_flat<STYLE, BONDS, FILT, FILT ? 12 : 16>, dim3(grid, parts), threads, s, a);
+    } else {
+        pdl_launch(k_pair_flat_split<STYLE, BONDS, FILT, FILT ? 16 : 20>, grid, threads, s, a);
+        pdl_launch(k_pair_flat_logsteps<STYLE, BONDS, FILT>, std::min(grid, 148 * (FILT ? 12 : 16)), threads, s, a);
+    }
+}
+
 template <int STYLE, bool BONDS>
-static void launch_pair2(int variant, int grid, cudaStream_t s, const StepArgs& a)
+static void launch_pair2(int variant, bool filt, int grid, cudaStream_t s, const StepArgs& a)
 {
     if (variant == 0) pdl_launch(k_pair<STYLE, BONDS>, grid, 256, s, a);
     else if (variant == 2) pdl_launch(k_pair_q<STYLE, BONDS, 4, true>, grid, 256, s, a);
     else if (variant == 3) pdl_launch(k_pair_q<STYLE, BONDS, 3, false>, grid, 256, s, a);
-    else if (variant == 4) pdl_launch(k_pair_flat<STYLE, BONDS, 4>, grid, 256, s, a);
-    else if (variant == 5) pdl_launch(k_pair_flat<STYLE, BONDS, 3>, grid, 256, s, a);
-    else if (variant == 6) pdl_launch(k_pair_flat<STYLE, BONDS, 4>, grid, 256, s, a);
-    else if (variant == 7) {
-        pdl_launch(k_pair_flat_split<STYLE, BONDS, 0, 6>, grid, 256, s, a);
-        pdl_launch(k_pair_flat_split<STYLE, BONDS, 1, 4>, grid, 256, s, a);
-    } else if (variant == 8) {
-        pdl_launch(k_pair_flat_split<STYLE, BONDS, 0, 5>, grid, 256, s, a);
-        pdl_launch(k_pair_flat_logsteps<STYLE, BONDS>, std::min(grid, 148 * 4), 256, s, a);
-    } else if (variant == 9) {
-        pdl_launch(k_pair_flat_split<STYLE, BONDS, 0, 5, true>, grid, 256, s, a);
-        pdl_launch(k_pair_flat_logsteps<STYLE, BONDS, true>, std::min(grid, 148 * 4), 256, s, a);
+    else if (variant >= 4 && variant <= 9) {
+        if (filt) launch_flat<STYLE, BONDS, true>(variant >= 7, s, a);
+        else launch_flat<STYLE, BONDS, false>(variant >= 7, s, a);
     } else if (variant == 10) {
         pdl_launch(k_pair_entry<STYLE, BONDS>, (a.nmax * (a.P >> 5) + 7) / 8, 256, s, a);
     }
@@ -799,18 +809,17 @@ static void launch_pair2(int variant, int grid, cudaStream_t s, const StepArgs& 
 
 // pair_variant 0: thread per particle; 1: warp pair-queue, i-side and
 // j-side forces by float4 reductions in L2, 4 blocks/SM; 2: warp pair-queue with the
-// i-side reduced through shared-memory atomics; 3: as 1 with 3 blocks/SM; 4: flattened
-// warp schedule, 4 blocks/SM; 5: flattened, 3 blocks/SM; 6: the flattened schedule with
-// the list build fused into it (DPD; mDPD falls back to 4); 7 and 8 (the default): the
-// flattened schedule as two launches, non-log steps without FP64 sums at 6 (7) or 5 (8)
-// blocks/SM, log steps at 4; 9: as 8 with the i-side forces summed per owner in the warp;
-// 10: one thread per list entry (small grids); 11 (DPD engines): no list, the cell-tile
-// kernel (kernels_tile.cuh) after the counting sort
+// i-side reduced through shared-memory atomics; 3: as 1 with 3 blocks/SM; 4, 5: flattened
+// warp schedule; 6: the flattened schedule with the list build fused into it (DPD; mDPD
+// falls back to 4); 7, 8 (the default) and 9: the flattened schedule as two launches,
+// non-log steps without FP64 sums at 40 warps/SM, log steps at 32; 10: one thread per list
+// entry (small grids); 11 (DPD engines): no list, the cell-tile kernel (kernels_tile.cuh)
+// after the counting sort
 template <int STYLE>
-static void launch_pair(int variant, bool bonds, int grid, cudaStream_t s, const StepArgs& a)
+static void launch_pair(int variant, bool bonds, bool filt, int grid, cudaStream_t s, const StepArgs& a)
 {
-    if (bonds) launch_pair2<STYLE, true>(variant, grid, s, a);
-    else launch_pair2<STYLE, false>(variant, grid, s, a);
+    if (bonds) launch_pair2<STYLE, true>(variant, filt, grid, s, a);
+    else launch_pair2<STYLE, false>(variant, filt, grid, s, a);
 }
 
 // The list-build chain; every kernel returns at once unless this phase's flag is set.
@@ -863,7 +872,10 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     const bool tiny = small && gp <= 148 && tune_.launch_mode != 3;
     // schedule 11: no neighbour list, the cell-tile kernel after the counting sort
     const bool tile = use_tile();
-    const int variant = tile ? 11 : (small && tune_.pair_variant == 8 ? (tiny ? 10 : 4) : tune_.pair_variant);
+    // a thread per list entry while its nmax warps per 32 slots fit the GPU at once (3000
+    // particles, nmax 96: 8.3 us against 10.2 for the flattened schedule; 24000: 30.9 against 14.3)
+    const bool entry = tiny && (int64_t)nmax_ * (P_ / 32) <= 148 * 64;
+    const int variant = tile ? 11 : (small && tune_.pair_variant == 8 ? (entry ? 10 : 4) : tune_.pair_variant);
     // schedule 6: the DPD list build runs inside the pair kernel
     const bool fused = variant == 6 && !any_mdpd_;
     enqueue_build(s, !fused && !tile,
@@ -887,12 +899,15 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
         }
     } else if (fused) {
         const BuildArgs ba = build_args(b_, P_, C_, nmax_, maxb_);
-        if (bonds_) pdl_launch(k_build_pair<true, 4>, gp, 256, s, sa, ba);
-        else pdl_launch(k_build_pair<false, 4>, gp, 256, s, sa, ba);
+        const int threads = DPD_FLAT_WARPS * 32, gw = (P_ + threads - 1) / threads;
+        if (bonds_ && filt_) pdl_launch(k_build_pair<true, true, 12>, gw, threads, s, sa, ba);
+        else if (bonds_) pdl_launch(k_build_pair<true, false, 16>, gw, threads, s, sa, ba);
+        else if (filt_) pdl_launch(k_build_pair<false, true, 12>, gw, threads, s, sa, ba);
+        else pdl_launch(k_build_pair<false, false, 16>, gw, threads, s, sa, ba);
     } else if (any_dpd_) {
-        launch_pair<0>(variant, bonds_, gp, s, sa);
+        launch_pair<0>(variant, bonds_, filt_, gp, s, sa);
     }
-    if (any_mdpd_) launch_pair<1>(variant, bonds_, gp, s, sa);
+    if (any_mdpd_) launch_pair<1>(variant, bonds_, filt_, gp, s, sa);
     if (ev1) cudaEventRecordWithFlags(ev1, s, cudaEventRecordExternal);
     if (nang_ > 0) pdl_launch(k_angle, (nang_ + 255) / 256, 256, s, sa, angle_tbl_, angle_coef_, angle_wrep_, nang_);
     if (rdf_) pdl_launch(k_rdf, gp, 256, s, sa);
@@ -1871,10 +1886,10 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
     const int pv = tune_.pair_variant == 11 ? 8 : tune_.pair_variant;
     if (d.style == 0) {
         if (peratom) k_pair_peratom<0><<<gp, 256, 0, stream_>>>(sa, pe_slot_, vir_slot_);
-        else launch_pair<0>(pv, false, gp, stream_, sa);
+        else launch_pair<0>(pv, false, filt_, gp, stream_, sa);
     } else {
         if (peratom) k_pair_peratom<1><<<gp, 256, 0, stream_>>>(sa, pe_slot_, vir_slot_);
-        else launch_pair<1>(pv, false, gp, stream_, sa);
+        else launch_pair<1>(pv, false, filt_, gp, stream_, sa);
     }
     k_aos_out<<<gp, 256, 0, stream_>>>(sa, d_force, d_pe, d_virial, pe_slot_, vir_slot_);
     k_aos_done<<<1, 1, 0, stream_>>>(b_.build_flag, b_.phase);

@@ -101,9 +101,9 @@ __global__ void __launch_bounds__(256) k_pair_peratom(StepArgs a, float* pe_slot
         if (!pair_force<STYLE, false>(crow, r2, dx, dy, dz, vi, vj, rho_i, rho_j, d.seed, step, gx, gy, gz, unused))
             continue;
         const int tj = type0_of(vj.w);
-        const float4 c1 = __ldg(crow + tj * 3 + 1);
+        const float4 c0 = __ldg(crow + tj * 3), c1 = __ldg(crow + tj * 3 + 1);
         const float r = sqrtf(r2);
-        const float wc = 1.0f - r * c1.x;
+        const float wc = 1.0f - r * c0.w;
         float pei, pej;
         if (STYLE == 0) {
             pei = pej = 0.5f * (c1.y * wc * wc);

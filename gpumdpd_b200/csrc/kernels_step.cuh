@@ -251,18 +251,17 @@ __device__ __forceinline__ bool pair_force(const float4* crow, float r2, float d
 {
     const int tj = type0_of(vj.w);
     const float4 c0 = __ldg(crow + tj * 3 + 0);
-    if (!(r2 <= c0.w)) return false;
     const float rinv = rsqrtf(r2);
     const float r = r2 * rinv;
-    if (r < 1.0e-10f) return false;
-    const float4 c1 = __ldg(crow + tj * 3 + 1);
+    const float wc = 1.0f - r * c0.w;
+    if (wc <= 0.0f || r < 1.0e-10f) return false;
     const float dot = dx * (vi.x - vj.x) + dy * (vi.y - vj.y) + dz * (vi.z - vj.z);
-    const float wc = 1.0f - r * c1.x;
     const int tagi = tag_of(vi.w), tagj = tag_of(vj.w);
     const float th = saru_theta((uint32_t)min(tagi, tagj), (uint32_t)max(tagi, tagj), seed, step);
     float fpair = c0.x * wc;
     float wd = 0.0f;
-    float4 c2;
+    float4 c1, c2;
+    if (LOG || STYLE == 1) c1 = __ldg(crow + tj * 3 + 1);
     if (STYLE == 1) {
         c2 = __ldg(crow + tj * 3 + 2);
         wd = fmaxf(1.0f - r * c1.w, 0.0f);
@@ -592,23 +591,6 @@ __global__ void __launch_bounds__(256, MINB) k_pair_q(StepArgs a)
 }
 
 // ---------------------------------------------------------------------------------
-// Pair force, flattened warp schedule.  The list entries of a warp's 32 particles are
-// taken as one sequence, particle by particle (lane-major); an exclusive scan of the
-// counts gives each particle's start.  Every iteration evaluates 32 consecutive entries,
-// one per lane, so all lanes are busy whatever the per-particle counts, with no
-// compaction queue; the owner of entry t is found by a 5-step binary search over the
-// starts.  The next chunk's entries are fetched while the current chunk is evaluated, and
-// the pos/vel gathers of a chunk are issued together, so each chunk waits for one L2
-// round trip.  Entries outside rc idle their lane for the Saru part, so this schedule
-// suits small skins (at skin 0 every listed pair is inside rc).  Both the i-side and
-// j-side forces go to L2 as float4 reductions.  FP64 log sums are flushed per warp, so
-// no block barrier is needed on non-log steps.
-// LOGM: 2 = any step; 0 = non-log steps only (no FP64 sums: fewer registers, more
-// warps per SM); 1 = log steps only.  0 and 1 are launched together, each returning at
-// once on the other kind of step.
-// SEG: the i-side forces of an iteration are summed per owner in registers first (the flat
-// entries of one owner sit in consecutive lanes: a segmented warp scan), so one float4
-// reduction per owner and iteration reaches L2 instead of one per pair.
 // Warp-level FP64 sums of a replica kept across several calls (grid-stride loops): added
 // to `tot` while the replica stays the same, flushed to the spread accumulators (one
 // atomic per field and warp) when it changes and at the end.
@@ -640,14 +622,48 @@ struct WarpAcc {
     }
 };
 
-template <int STYLE, bool BONDS, int LOGM = 2, bool SEG = false>
-__device__ __forceinline__ void pair_flat_warp(const StepArgs& a, const int s, WarpAcc<8>* keep = nullptr)
+// Pair force, flattened warp schedule.  The list entries of a warp's 32 particles are
+// taken as one sequence, particle by particle, and cut into 32 runs of equal length, one
+// per lane: every lane evaluates one pair per iteration whatever the per-particle counts,
+// and sums the forces of the particle its run is in (the owner) in registers.  The owner's
+// sum goes to L2 as a float4 reduction where the run leaves the particle, so a warp sends
+// about 32 + 31 owner sums instead of one per pair; the other side of each pair is one
+// float4 reduction.  A 32-lane float4 reduction takes 32 wavefronts of the L1 data pipe:
+// with one per side and pair they were over half of its load (72% busy on a 648k melt at
+// skin 0; now 66% in 11% less time).  The owner of a run's first entry is found by a 5-step
+// binary search over the scanned counts, later ones by stepping.  What bounds it now: the
+// latency of the dependent gathers (list entry, then position and velocity: half of the
+// stalls) and the integer pipe (48% busy; the random number alone is 174 clocks per 32
+// pairs and scheduler).  3M melt, skin 0: 337 -> 297 us a step; the next pair's gathers held
+// in registers during the current one: 320; the entries staged in shared memory first: 330.
+// FILT: the list holds entries outside the largest cutoff (a skin, or a global cutoff above
+// it).  Each lane then first filters its own particle's entries, 4 gathers in flight, into
+// its column of a shared queue, and the runs are cut from the queued pairs, so the random
+// number and the force run with all lanes on pairs that need them (at skin 0.3 and rc 1
+// these are 46% of the entries); a lane whose column is full ends the round early, and the
+// rest is filtered in the next one.  648k melt, skin 0.3: 136 -> 115 us a step; 384k
+// many-body slab: 161 -> 114.
+// part, nparts: the entries [n part/nparts, n (part+1)/nparts) of each particle, for small
+// grids, where several warps share 32 particles; bonds go with part 0.
+// LOGM: 2 = any step; 0 = non-log steps only (no FP64 sums: fewer registers, more
+// warps per SM); 1 = log steps only.  0 and 1 are launched together, each returning at
+// once on the other kind of step.  FP64 log sums are flushed per warp, so no block barrier
+// is needed.  FILT is compiled for 32 warps per SM (64 registers; 40 spill and take 141 us
+// at 648k), the others for 40.
+#define DPD_FLAT_WARPS 2  // warps per block of the flattened kernels
+#define DPD_FLAT_COL 16   // queued entries per particle and round
+template <int STYLE, bool BONDS, bool FILT, int LOGM = 2>
+__device__ __forceinline__ void pair_flat_warp(const StepArgs& a, const int s, WarpAcc<8>* keep = nullptr,
+                                               const int part = 0, const int nparts = 1)
 {
-    __shared__ int s_start[8][33];
-    __shared__ float4 s_pi[8][32];
-    __shared__ float4 s_vi[8][32];
-    __shared__ float s_rho[8][32];
-    __shared__ float4 tab[8][27];
+    __shared__ int s_start[DPD_FLAT_WARPS][33];
+    __shared__ int s_off[DPD_FLAT_WARPS][32];
+    __shared__ float4 s_pi[DPD_FLAT_WARPS][32];
+    __shared__ float4 s_vi[DPD_FLAT_WARPS][32];
+    __shared__ float s_rho[STYLE == 1 ? DPD_FLAT_WARPS : 1][32];
+    __shared__ float s_fb[BONDS ? DPD_FLAT_WARPS : 1][3][32];  // bond forces: where an owner's sum starts
+    __shared__ int s_q[FILT ? DPD_FLAT_WARPS : 1][DPD_FLAT_COL * 32];
+    __shared__ float4 tab[DPD_FLAT_WARPS][27];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if ((s & ~31) >= a.P) return;  // whole warp beyond the slots
     const int r = a.warp_rep[s >> 5];
@@ -673,130 +689,172 @@ __device__ __forceinline__ void pair_flat_warp(const StepArgs& a, const int s, W
     const float4* pos = a.buf.pos[par];
     const float4* vel = a.buf.vel[par];
     fill_shift(tab[warp], d, lane);
-    float4 pi = make_float4(0, 0, 0, 0), vi = make_float4(0, 0, 0, 0);
-    float rho_i = 0.0f;
-    int n = 0;
+    float4 pi = make_float4(0, 0, 0, 0);
+    int k = 0, kend = 0;  // this part's entries of the lane's particle still to be taken
     if (work) {
         pi = pos[s];
-        vi = vel[s];
-        if (STYLE == 1) rho_i = a.rho[s];
-        n = min(a.ncount[s], a.nmax);
+        s_vi[warp][lane] = vel[s];
+        if (STYLE == 1) s_rho[warp][lane] = a.rho[s];
+        kend = min(a.ncount[s], a.nmax);
+        if (nparts > 1) {
+            k = kend * part / nparts;
+            kend = kend * (part + 1) / nparts;
+        }
     }
     s_pi[warp][lane] = pi;
-    s_vi[warp][lane] = vi;
-    s_rho[warp][lane] = rho_i;
-    int incl = n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+    if (BONDS) {
+        float bx = 0.0f, by = 0.0f, bz = 0.0f;
+        if (work && part == 0) {
+            if (log) bond_loop<true>(a, d, pos, a.buf.bonds[par], r, s, pi, bx, by, bz, accv);
+            else bond_loop<false>(a, d, pos, a.buf.bonds[par], r, s, pi, bx, by, bz, accv);
+        }
+        s_fb[warp][0][lane] = bx;
+        s_fb[warp][1][lane] = by;
+        s_fb[warp][2][lane] = bz;
     }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    s_start[warp][lane] = incl - n;
-    if (lane == 31) s_start[warp][32] = total;
-    __syncwarp();
     const int* wl = a.nlist + (size_t)(s >> 5) * a.nmax * 32;
     const float rcmax2 = d.rcmax2;
     const float4* cbase = a.coeff + d.coeff_off;
     const int nt = d.ntypes;
     const uint32_t seed = d.seed;
     const int wbase = s & ~31;
-    // owner lane and list entry of flat entry t (t < total)
-    auto locate = [&](int t, int& l, int& ent) {
-        int lo = 0;  // largest l with start[l] <= t (empty particles share a start)
+    __syncwarp();
+    bool first = true;
+    do {
+        // this round's entries: the list itself, or the lane's filtered column
+        int c = kend - k;
+        int kb = k;  // where the entries of the lane's particle begin in `src`
+        if (FILT) {
+            c = 0;
+            kb = 0;
+            int* col = s_q[warp] + lane;
+            // a round ends when a column might not take 4 more entries
+            while (__any_sync(0xffffffffu, k < kend) && !__any_sync(0xffffffffu, c > DPD_FLAT_COL - 4)) {
+                int ee[4];
+                float4 pp[4];
 #pragma unroll
-        for (int stp = 16; stp >= 1; stp >>= 1)
-            if (s_start[warp][lo + stp] <= t) lo += stp;
-        l = lo;
-        // a plain load: the fused kernel reads entries its own warp has just written
-        ent = wl[(size_t)(t - s_start[warp][lo]) * 32 + lo];
-    };
-    int l_nx = 0, ent_nx = 0;
-    if (lane < total) locate(lane, l_nx, ent_nx);
-    for (int t0 = 0; t0 < total; t0 += 32) {
-        const bool valid = t0 + lane < total;
-        const int l = l_nx, ent = ent_nx;
-        float4 pj = make_float4(0, 0, 0, 0), vj = make_float4(0, 0, 0, 0);
-        float rho_j = 0.0f;
-        const int j = ent & DPD_J_MASK;
-        if (valid) {
-            pj = __ldg(pos + j);
-            vj = __ldg(vel + j);
-            if (STYLE == 1) rho_j = __ldg(a.rho + j);
-        }
-        if (t0 + 32 + lane < total) locate(t0 + 32 + lane, l_nx, ent_nx);
-        float ix = 0.0f, iy = 0.0f, iz = 0.0f;
-        if (valid) {
-            const float4 pil = s_pi[warp][l];
-            float dx, dy, dz;
-            pair_disp(tab[warp], ent, pil, pj, dx, dy, dz);
-            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-            if (r2 <= rcmax2) {
-                const float4 vv = s_vi[warp][l];
-                const float4* crow = cbase + type0_of(vv.w) * nt * 3;
-                float fx, fy, fz;
-                const bool ok = log ? pair_force<STYLE, true>(crow, r2, dx, dy, dz, vv, vj, s_rho[warp][l], rho_j, seed, step, fx, fy, fz, accv)
-                                    : pair_force<STYLE, false>(crow, r2, dx, dy, dz, vv, vj, s_rho[warp][l], rho_j, seed, step, fx, fy, fz, accv);
-                if (ok) {
-                    atomicAdd(&a.force4[j], make_float4(-fx, -fy, -fz, 0.0f));
-                    if (SEG) {
-                        ix = fx;
-                        iy = fy;
-                        iz = fz;
-                    } else {
-                        atomicAdd(&a.force4[wbase + l], make_float4(fx, fy, fz, 0.0f));
+                for (int u = 0; u < 4; u++) ee[u] = k + u < kend ? wl[(size_t)(k + u) * 32 + lane] : 0;
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (k + u < kend) pp[u] = __ldg(pos + (ee[u] & DPD_J_MASK));
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (k + u < kend) {
+                        float dx, dy, dz;
+                        pair_disp(tab[warp], ee[u], pi, pp[u], dx, dy, dz);
+                        const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+                        if (r2 <= rcmax2) {
+                            col[c * 32] = ee[u];
+                            c++;
+                        }
                     }
-                }
+                k += 4;
             }
         }
-        if (SEG) {
-            // lanes past the end get keys of their own: they never join a segment
-            const int key = valid ? l : 32 + lane;
+        int incl = c;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const float tx = __shfl_up_sync(0xffffffffu, ix, o);
-                const float ty = __shfl_up_sync(0xffffffffu, iy, o);
-                const float tz = __shfl_up_sync(0xffffffffu, iz, o);
-                const int tk = __shfl_up_sync(0xffffffffu, key, o);
-                if (lane >= o && tk == key) {
-                    ix += tx;
-                    iy += ty;
-                    iz += tz;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        s_start[warp][lane] = incl - c;
+        s_off[warp][lane] = (kb - (incl - c)) * 32 + lane;  // entry t of the sequence: src[t * 32 + off]
+        if (lane == 31) s_start[warp][32] = total;
+        // a particle without pairs in this round sends its bond force itself
+        if (BONDS && first && c == 0 && work && part == 0)
+            atomicAdd(&a.force4[s], make_float4(s_fb[warp][0][lane], s_fb[warp][1][lane], s_fb[warp][2][lane], 0.0f));
+        __syncwarp();
+        const int* src = FILT ? s_q[warp] : wl;
+        const int per = (total + 31) >> 5;
+        int t = lane * per;
+        const int te = min(t + per, total);
+        int l = 0, nxt = 0, off = 0;
+        float4 pl = make_float4(0, 0, 0, 0), vl = make_float4(0, 0, 0, 0);
+        float rho_l = 0.0f, fx = 0.0f, fy = 0.0f, fz = 0.0f;
+        if (t < te) {
+            // the largest l with start[l] <= t (particles without entries share a start)
+#pragma unroll
+            for (int stp = 16; stp >= 1; stp >>= 1)
+                if (s_start[warp][l + stp] <= t) l += stp;
+            nxt = s_start[warp][l + 1];
+            off = s_off[warp][l];
+            pl = s_pi[warp][l];
+            vl = s_vi[warp][l];
+            if (STYLE == 1) rho_l = s_rho[warp][l];
+            if (BONDS && first && t == s_start[warp][l]) {
+                fx = s_fb[warp][0][l];
+                fy = s_fb[warp][1][l];
+                fz = s_fb[warp][2][l];
+            }
+        }
+        for (int it = 0; it < per; it++, t++) {
+            if (t >= te) break;
+            if (t == nxt) {
+                // the run leaves its particle: the sum so far, then the next one with entries
+                atomicAdd(&a.force4[wbase + l], make_float4(fx, fy, fz, 0.0f));
+                do {
+                    l++;
+                    nxt = s_start[warp][l + 1];
+                } while (nxt == t);
+                off = s_off[warp][l];
+                pl = s_pi[warp][l];
+                vl = s_vi[warp][l];
+                if (STYLE == 1) rho_l = s_rho[warp][l];
+                fx = fy = fz = 0.0f;
+                if (BONDS && first) {
+                    fx = s_fb[warp][0][l];
+                    fy = s_fb[warp][1][l];
+                    fz = s_fb[warp][2][l];
                 }
             }
-            const int nk = __shfl_down_sync(0xffffffffu, key, 1);
-            if (valid && (lane == 31 || nk != key) && (ix != 0.0f || iy != 0.0f || iz != 0.0f))
-                atomicAdd(&a.force4[wbase + l], make_float4(ix, iy, iz, 0.0f));
+            const int ent = src[t * 32 + off];
+            const int j = ent & DPD_J_MASK;
+            const float4 pj = __ldg(pos + j), vj = __ldg(vel + j);
+            const float rho_j = STYLE == 1 ? __ldg(a.rho + j) : 0.0f;
+            float dx, dy, dz;
+            pair_disp(tab[warp], ent, pl, pj, dx, dy, dz);
+            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+            if (FILT || r2 <= rcmax2) {
+                const float4* crow = cbase + type0_of(vl.w) * nt * 3;
+                float gx, gy, gz;
+                const bool ok = log ? pair_force<STYLE, true>(crow, r2, dx, dy, dz, vl, vj, rho_l, rho_j, seed, step, gx, gy, gz, accv)
+                                    : pair_force<STYLE, false>(crow, r2, dx, dy, dz, vl, vj, rho_l, rho_j, seed, step, gx, gy, gz, accv);
+                if (ok) {
+                    atomicAdd(&a.force4[j], make_float4(-gx, -gy, -gz, 0.0f));
+                    fx += gx;
+                    fy += gy;
+                    fz += gz;
+                }
+            }
         }
-    }
-    if (BONDS && work) {
-        float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-        if (log) bond_loop<true>(a, d, pos, a.buf.bonds[par], r, s, pi, fx, fy, fz, accv);
-        else bond_loop<false>(a, d, pos, a.buf.bonds[par], r, s, pi, fx, fy, fz, accv);
-        atomicAdd(&a.force4[s], make_float4(fx, fy, fz, 0.0f));
-    }
+        if (lane * per < te) atomicAdd(&a.force4[wbase + l], make_float4(fx, fy, fz, 0.0f));
+        first = false;
+        __syncwarp();  // the shared slots are reused by the next round
+    } while (FILT && __any_sync(0xffffffffu, k < kend));
     if (log && !keep) acc_flush_warp<8>(accv, fields, r, a.acc);
 }
 
-template <int STYLE, bool BONDS, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_pair_flat(StepArgs a)
+// any step in one launch; grid (blocks of DPD_FLAT_WARPS x 32 slots, parts)
+template <int STYLE, bool BONDS, bool FILT, int MINB>
+__global__ void __launch_bounds__(DPD_FLAT_WARPS * 32, MINB) k_pair_flat(StepArgs a)
 {
     griddep_wait();
-    pair_flat_warp<STYLE, BONDS>(a, blockIdx.x * blockDim.x + threadIdx.x);
+    pair_flat_warp<STYLE, BONDS, FILT>(a, blockIdx.x * blockDim.x + threadIdx.x, nullptr, blockIdx.y, gridDim.y);
 }
 
-template <int STYLE, bool BONDS, int LOGM, int MINB, bool SEG = false>
-__global__ void __launch_bounds__(256, MINB) k_pair_flat_split(StepArgs a)
+template <int STYLE, bool BONDS, bool FILT, int MINB>
+__global__ void __launch_bounds__(DPD_FLAT_WARPS * 32, MINB) k_pair_flat_split(StepArgs a)
 {
     griddep_wait();
-    pair_flat_warp<STYLE, BONDS, LOGM, SEG>(a, blockIdx.x * blockDim.x + threadIdx.x);
+    pair_flat_warp<STYLE, BONDS, FILT, 0>(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // The log-step half of the split schedule as a small grid-stride launch: every block
 // first checks whether any replica logs this step (the common answer is no, and then the
 // launch costs one wave of tiny blocks instead of a full grid of early exits).
-template <int STYLE, bool BONDS, bool SEG = false>
-__global__ void __launch_bounds__(256, 4) k_pair_flat_logsteps(StepArgs a)
+template <int STYLE, bool BONDS, bool FILT>
+__global__ void __launch_bounds__(DPD_FLAT_WARPS * 32, FILT ? 12 : 16) k_pair_flat_logsteps(StepArgs a)
 {
     griddep_wait();
     int any = 0;
@@ -805,11 +863,11 @@ __global__ void __launch_bounds__(256, 4) k_pair_flat_logsteps(StepArgs a)
         any |= rep_active(st) && (st.step % (uint32_t)a.reps[r].log_f) == 0u;
     }
     if (!__syncthreads_or(any)) return;
-    const int nvb = (a.P + 255) / 256;
+    const int nvb = (a.P + blockDim.x - 1) / blockDim.x;
     // the warp's sums over its virtual blocks, flushed once per replica
     WarpAcc<8> keep;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-        pair_flat_warp<STYLE, BONDS, 1, SEG>(a, vb * 256 + threadIdx.x, &keep);
+        pair_flat_warp<STYLE, BONDS, FILT, 1>(a, vb * blockDim.x + threadIdx.x, &keep);
         __syncwarp();  // the warp's shared slots are reused by the next virtual block
     }
     const int fields[8] = {ACC_PAIR_PE, ACC_BOND_PE, ACC_VIR + 0, ACC_VIR + 1,
@@ -822,15 +880,15 @@ __global__ void __launch_bounds__(256, 4) k_pair_flat_logsteps(StepArgs a)
 // (the list of the build kernel, bit for bit), then evaluates those pairs at once, while
 // the neighbours' positions are still in L1; on other steps it is the flattened pair
 // kernel.  One launch instead of two, and the list is read back from L1/L2.
-template <bool BONDS, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_build_pair(StepArgs a, BuildArgs b)
+template <bool BONDS, bool FILT, int MINB>
+__global__ void __launch_bounds__(DPD_FLAT_WARPS * 32, MINB) k_build_pair(StepArgs a, BuildArgs b)
 {
     griddep_wait();
     if (build_on(b)) {
         build_nlist_slot(b, blockIdx.x * blockDim.x + threadIdx.x);
         __syncwarp();
     }
-    pair_flat_warp<0, BONDS>(a, blockIdx.x * blockDim.x + threadIdx.x);
+    pair_flat_warp<0, BONDS, FILT>(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------------
