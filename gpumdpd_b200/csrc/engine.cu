@@ -54,8 +54,7 @@ Engine::~Engine()
     if (stream_) cudaStreamSynchronize(stream_);
     for (void* p : allocs_) cudaFreeAsync(p, stream_);
     if (stream_) cudaStreamSynchronize(stream_);
-    for (void* p : {(void*)h_pos_, (void*)h_vel_, (void*)h_frc_, (void*)h_img_})
-        if (p) cudaFreeHost(p);
+    if (h_block_) cudaFreeHost(h_block_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -548,13 +547,21 @@ int Engine::alloc_and_upload()
     return DPD_OK;
 }
 
+#define DPD_ROWS_PINNED 64  // thermo rows that a read-back stages in pinned memory
+
 int Engine::staging()
 {
-    if (h_pos_) return DPD_OK;
-    CK(cudaMallocHost((void**)&h_pos_, sizeof(float4) * P_));
-    CK(cudaMallocHost((void**)&h_vel_, sizeof(float4) * P_));
-    CK(cudaMallocHost((void**)&h_frc_, sizeof(float4) * P_));
-    CK(cudaMallocHost((void**)&h_img_, sizeof(int4) * P_));
+    if (h_block_) return DPD_OK;
+    const size_t arr = sizeof(float4) * (size_t)P_;
+    const size_t rs = (sizeof(RepState) * reps_.size() + 127) / 128 * 128;
+    // 512: the rows of a state read-back start on 128-byte lines
+    CK(cudaMallocHost((void**)&h_block_, 4 * arr + 512 + rs + sizeof(double) * (DPD_ROWS_PINNED * DPD_THERMO_FIELDS + 1)));
+    h_pos_ = (float4*)h_block_;
+    h_vel_ = h_pos_ + P_;
+    h_frc_ = h_vel_ + P_;
+    h_img_ = (int4*)(h_frc_ + P_);
+    h_rs_ = (RepState*)(h_block_ + 4 * arr + 512);
+    h_rows_ = (double*)((char*)h_rs_ + rs);
     return DPD_OK;
 }
 
@@ -1142,8 +1149,9 @@ int Engine::run(uint32_t nsteps)
 int Engine::read_rstate(std::vector<RepState>& st)
 {
     st.resize(reps_.size());
-    CK(cudaMemcpyAsync(st.data(), b_.rstate, sizeof(RepState) * st.size(), cudaMemcpyDeviceToHost, stream_));
+    CK(cudaMemcpyAsync(h_rs_, b_.rstate, sizeof(RepState) * st.size(), cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
+    memcpy(st.data(), h_rs_, sizeof(RepState) * st.size());
     return DPD_OK;
 }
 
@@ -1155,11 +1163,10 @@ int Engine::rstate_async(RepState* host)
 
 int Engine::sync_and_check()
 {
-    CK(cudaStreamSynchronize(stream_));
-    CK(cudaGetLastError());
     std::vector<RepState> st;
     int e = read_rstate(st);
     if (e) return e;
+    CK(cudaGetLastError());
     for (size_t r = 0; r < st.size(); r++) {
         const int code = status_error(st[r].status, (int)r);
         if (code) return code;
@@ -1354,19 +1361,32 @@ int64_t Engine::total_atoms() const
 int Engine::get_thermo(int rep, dpd_thermo* rows, int max_rows, int* n_rows)
 {
     if (rep < 0 || rep >= (int)reps_.size()) return DPD_E_ARG;
-    std::vector<RepState> st;
-    int e = read_rstate(st);
-    if (e) return e;
-    const int nlog = st[rep].nlog;
-    const int avail = std::min(nlog, DPD_RING_ROWS);
-    const int n = std::min(avail, max_rows);
-    std::vector<double> ring((size_t)DPD_RING_ROWS * DPD_THERMO_FIELDS);
-    CK(cudaMemcpyAsync(ring.data(), b_.ring + (size_t)rep * DPD_RING_ROWS * DPD_THERMO_FIELDS,
-                       sizeof(double) * ring.size(), cudaMemcpyDeviceToHost, stream_));
-    CK(cudaStreamSynchronize(stream_));
+    const double* got = h_rows_;
+    std::vector<double> ring;
+    int n = 0, first = 0;
+    if (max_rows <= DPD_ROWS_PINNED) {
+        int* count = (int*)(h_rows_ + DPD_ROWS_PINNED * DPD_THERMO_FIELDS);
+        k_thermo_out<<<1, 256, 0, stream_>>>(step_args(b_, P_, nmax_, maxb_, (int)reps_.size()), rep, std::max(max_rows, 0),
+                                             count, h_rows_);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(stream_));
+        n = *count;
+    } else {
+        std::vector<RepState> st;
+        int e = read_rstate(st);
+        if (e) return e;
+        const int nlog = st[rep].nlog;
+        n = std::min(std::min(nlog, DPD_RING_ROWS), max_rows);
+        first = (nlog - n) % DPD_RING_ROWS;
+        // the ring up to the rows in use
+        ring.resize((size_t)std::min(nlog, DPD_RING_ROWS) * DPD_THERMO_FIELDS);
+        CK(cudaMemcpyAsync(ring.data(), b_.ring + (size_t)rep * DPD_RING_ROWS * DPD_THERMO_FIELDS,
+                           sizeof(double) * ring.size(), cudaMemcpyDeviceToHost, stream_));
+        CK(cudaStreamSynchronize(stream_));
+        got = ring.data();
+    }
     for (int k = 0; k < n; k++) {
-        const int idx = (nlog - n + k) % DPD_RING_ROWS;
-        const double* row = ring.data() + (size_t)idx * DPD_THERMO_FIELDS;
+        const double* row = got + (size_t)((first + k) % DPD_RING_ROWS) * DPD_THERMO_FIELDS;
         dpd_thermo& t = rows[k];
         t.step = (int64_t)row[0];
         t.temp = row[1];
@@ -1444,31 +1464,50 @@ int Engine::get_state(int rep, double* x, double* v, int* image, double* f)
     if (rep < 0 || rep >= (int)reps_.size()) return DPD_E_ARG;
     const RepDesc& d = reps_[rep].desc;
     const Replica& R = reps_[rep];
-    const int ns = d.p_cap_end - d.p_begin;
+    const int64_t n = d.n_real;
     int st = staging();
     if (st) return st;
-    float4* pos = h_pos_;
-    float4* vel = h_vel_;
-    float4* frc = h_frc_;
-    int4* img = h_img_;
-    const int par = cur_parity();
-    if (par < 0) return cuda_fail(cudaGetLastError(), "cudaMemcpy(parity)");
-    CK(cudaMemcpyAsync(vel, b_.vel[par] + d.p_begin, sizeof(float4) * ns, cudaMemcpyDeviceToHost, stream_));
-    if (x || image) {
-        CK(cudaMemcpyAsync(pos, b_.pos[par] + d.p_begin, sizeof(float4) * ns, cudaMemcpyDeviceToHost, stream_));
-        CK(cudaMemcpyAsync(img, b_.img + d.tag_base, sizeof(int4) * d.n_real, cudaMemcpyDeviceToHost, stream_));
-    }
-    if (f) CK(cudaMemcpyAsync(frc, b_.force4 + d.p_begin, sizeof(float4) * ns, cudaMemcpyDeviceToHost, stream_));
+    // rows by tag in the pinned block, each array from a 128-byte line: 60 of its 64 bytes
+    // per slot
+    auto line = [](size_t b) { return (b + 127) / 128 * 128; };
+    StateOut o;
+    for (int q = 0; q < 3; q++) o.L[q] = R.box_len[q];
+    size_t at = 0;
+    o.x = x ? (double*)(h_block_ + at) : nullptr;
+    if (x) at += line(sizeof(double) * 3 * n);
+    o.v = v ? (float*)(h_block_ + at) : nullptr;
+    if (v) at += line(sizeof(float) * 3 * n);
+    o.f = f ? (float*)(h_block_ + at) : nullptr;
+    if (f) at += line(sizeof(float) * 3 * n);
+    o.image = image ? (int*)(h_block_ + at) : nullptr;
+    o.bad = (int*)h_rows_;
+    *o.bad = 0;
+    k_state_out<<<(int)((n + 255) / 256), 256, 0, stream_>>>(step_args(b_, P_, nmax_, maxb_, (int)reps_.size()), rep, o);
+    CK(cudaGetLastError());
     // a spring's share of the force (post_force adds it to the force array the reference
     // dumps, src/fix/fix_spring.cu:350-370); the engine adds it inside the half kicks
     FixOut fo{};
     const bool spring = f && b_.fixo && R.ff.spring.on && R.ff.spring.mask;
     if (spring) CK(cudaMemcpyAsync(&fo, b_.fixo + rep, sizeof(FixOut), cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
-    if (!slots_to_tags(rep, pos, vel, img, frc, spring ? fo.spring_a : nullptr, x, v, image, f)) {
+    if (*o.bad) {
         err = "corrupt tag in device state";
         return DPD_E_STATE;
     }
+    parallel_for(3 * n, [&](int64_t k0, int64_t k1) {
+        if (x) memcpy(x + k0, o.x + k0, sizeof(double) * (k1 - k0));
+        if (image) memcpy(image + k0, o.image + k0, sizeof(int) * (k1 - k0));
+        if (v)
+            for (int64_t k = k0; k < k1; k++) v[k] = o.v[k];
+        if (f)
+            for (int64_t k = k0; k < k1; k++) f[k] = o.f[k];
+    }, 131072);
+    if (spring)
+        for (int64_t i = 0; i < n; i++) {
+            const int t0 = R.sys.type[i] - 1;
+            if ((R.ff.spring.mask >> t0) & 1u)
+                for (int q = 0; q < 3; q++) f[3 * i + q] += (double)fo.spring_a[q] * R.sys.masses[t0];
+        }
     return DPD_OK;
 }
 

@@ -18,11 +18,12 @@ struct StepArgs;  // kernels_step.cuh
 namespace dpd {
 
 // Host loop over [0, n) split across hardware threads (state conversion of millions of
-// particles on every upload/download).
+// particles on every upload/download); `grain`: fewest items worth a thread of their own.
 template <class F>
-inline void parallel_for(int64_t n, F fn)
+inline void parallel_for(int64_t n, F fn, int64_t grain = 1)
 {
     int nt = (int)std::min<int64_t>(std::max(1u, std::thread::hardware_concurrency()), 32);
+    nt = (int)std::max<int64_t>(1, std::min<int64_t>(nt, n / grain));
     if (n < 65536) nt = 1;
     std::vector<std::thread> th;
     for (int t = 1; t < nt; t++) th.emplace_back([=] { fn(n * t / nt, n * (t + 1) / nt); });
@@ -216,8 +217,13 @@ private:
     bool ranks_dirty_ = false;  // new cell ranks (a changed cell order) wait for the next run
     uint32_t next_step_ = 0;
     std::vector<void*> allocs_;
-    float4 *h_pos_ = nullptr, *h_vel_ = nullptr, *h_frc_ = nullptr;  // pinned staging
+    char* h_block_ = nullptr;  // pinned staging, one block: the four arrays below (64 B per
+                               // slot, also the rows of a state read-back), the replica
+                               // states, and rows of a thermo read-back
+    float4 *h_pos_ = nullptr, *h_vel_ = nullptr, *h_frc_ = nullptr;
     int4* h_img_ = nullptr;
+    RepState* h_rs_ = nullptr;
+    double* h_rows_ = nullptr;
     int2* bonds_tag_ = nullptr;  // bond partner table in tag order (device)
     int4* angle_tbl_ = nullptr;   // angles: {coef index or -1, global tags i, j, k}
     float4* angle_coef_ = nullptr;  // {k, theta0 in radians, cos, sin theta0} per replica and angle type
