@@ -2,14 +2,14 @@
 //
 // State lives in tag order as wrapped FP64 positions, velocities, forces and image counters.
 // Each step: the initial half kick and drift with wrapping (src/fix/fix_nve.cu:42-86), a
-// cell grid of fixed-capacity cells (atomic append, then each cell sorted by index so the
-// summation order is fixed), the mDPD density pass (src/force/pair_mdpd.cu:253-297), the
-// force pass, the final half kick (src/fix/fix_nve.cu:131-149) and on logged steps a
-// fixed-order reduction of the thermo sums (src/compute/thermo.cu:240-246,301-303,422-434,
-// 506-517).  The force pass gives one warp per atom all its pairs from both sides (the
-// 27 cells' candidates filtered 32 at a time, the pairs inside the cutoff evaluated 32 at
-// a time), its bonds and its angles, summed by a fixed butterfly, so no atomics touch the
-// forces and runs repeat bit for bit.
+// cell grid of fixed-capacity cells (indices appended by atomics, then each cell's records
+// written in index order so the summation order is fixed), the mDPD density pass
+// (src/force/pair_mdpd.cu:253-297), the force pass, the final half kick
+// (src/fix/fix_nve.cu:131-149) and on logged steps a fixed-order reduction of the thermo sums
+// (src/compute/thermo.cu:240-246,301-303,422-434,506-517).  The force pass gives one warp all
+// pairs of a cell's atoms from both sides (the 27 cells' candidates staged once, the pairs
+// inside the cutoff evaluated 32 at a time), their bonds and angles, summed by fixed trees, so
+// no atomics touch the forces and runs repeat bit for bit.
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -36,7 +36,8 @@ struct F64Args {
     const double *coeff, *mass, *bondc, *anglec;
     double *x, *v, *f, *rho, *q;
     int *img, *type, *cnt, *status;
-    double4* crec;  // cell records: position and atom index (exact in a double), cap per cell
+    int* craw;      // atom indices appended to each cell, cap per cell
+    double4* crec;  // cell records in index order: position and atom index (rec_index)
     int* ccode;  // each atom's cell as cx | cy << 10 | cz << 20, written by the binning
     const int *bstart, *astart;
     const int2* bent;
@@ -47,8 +48,12 @@ struct F64Args {
 __device__ __forceinline__ double min_image(double d, double L)
 {
     const double h = 0.5 * L;
-    return d - L * (double)((d >= h) - (d < -h));
+    return d - (d >= h ? L : (d < -h ? -L : 0.0));
 }
+
+// the atom index of a cell record, kept as the bits of its fourth word
+__device__ __forceinline__ double rec_word(int i) { return __longlong_as_double((long long)i); }
+__device__ __forceinline__ int rec_index(const double4& r) { return (int)__double_as_longlong(r.w); }
 
 // triangular type-pair index, src/force/pair_dpd.cu:134 (types 1-based, result 0-based)
 __device__ __forceinline__ int tri(int ti, int tj, int nt)
@@ -82,26 +87,26 @@ __global__ void k64_bin(F64Args a)
     const int cell = cell_of(a, a.x + 3 * i, c);
     a.ccode[i] = c[0] | (c[1] << 10) | (c[2] << 20);
     const int k = atomicAdd(a.cnt + cell, 1);
-    if (k < a.cap)
-        a.crec[(size_t)cell * a.cap + k] = make_double4(a.x[3 * i], a.x[3 * i + 1], a.x[3 * i + 2], (double)i);
+    if (k < a.cap) a.craw[(size_t)cell * a.cap + k] = i;
     else atomicOr(a.status, F64_CELL_OVERFLOW);
 }
 
-// each cell's records in atom-index order: the pair sums then run in a fixed order
-__global__ void k64_sort_cells(F64Args a, int ncell)
+// each cell's records in atom-index order, so the pair sums run in a fixed order: 8 lanes per
+// cell rank its indices (a record's place is the number of smaller indices) and gather the
+// records
+__global__ void __launch_bounds__(256) k64_sort_cells(F64Args a, int ncell)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = g >> 3;
     if (c >= ncell) return;
-    double4* l = a.crec + (size_t)c * a.cap;
+    const int* raw = a.craw + (size_t)c * a.cap;
     const int m = min(a.cnt[c], a.cap);
-    for (int p = 1; p < m; p++) {
-        const double4 v = l[p];
-        int q = p - 1;
-        while (q >= 0 && l[q].w > v.w) {
-            l[q + 1] = l[q];
-            q--;
-        }
-        l[q + 1] = v;
+    for (int k = g & 7; k < m; k += 8) {
+        const int i = raw[k];
+        int place = 0;
+        for (int q = 0; q < m; q++) place += raw[q] < i;
+        const size_t to = (size_t)c * a.cap + place;
+        a.crec[to] = make_double4(a.x[3 * i], a.x[3 * i + 1], a.x[3 * i + 2], rec_word(i));
     }
 }
 
@@ -122,7 +127,7 @@ __device__ __forceinline__ void for_cell(const F64Args& a, int i, int c, F&& fn)
     const int m = min(a.cnt[cell], a.cap);
     for (int p = 0; p < m; p++) {
         const double4 rj = l[p];
-        const int j = (int)rj.w;
+        const int j = rec_index(rj);
         if (j == i) continue;
         const double dx = min_image(xi - rj.x, a.L[0]);
         const double dy = min_image(yi - rj.y, a.L[1]);
@@ -161,88 +166,127 @@ __global__ void __launch_bounds__(256) k64_density(F64Args a)
     if (lane == 0) a.rho[i] = rho;
 }
 
-// Forces on atom i, one warp per atom.  The records of the 27 cells around the atom
-// (src/force/pair_dpd.cu:292-403, pair_mdpd.cu:399-521) are taken 32 at a time as one
-// sequence, cell by cell in a fixed order and each cell's records in index order: each
-// lane tests one candidate, the pairs inside the largest cutoff are queued in the warp's
-// shared ring in ballot order, and whenever 32 are queued every lane evaluates one (the
-// Saru random force, the FP64 force) into its own partial sums -- a fixed assignment of
-// pairs to lanes, so the sums repeat bit for bit.  The lanes also share out the atom's
-// bonds (src/force/bond_harmonic.cu:208-268; FENE + WCA as the FP32 engine) and harmonic
-// angles (src/force/angle_harmonic.cu:187-270), and a fixed butterfly sums the lanes.  On
-// logged steps the atom's share of the energies and of the virial: half of each pair and
-// bond, a third of each angle, as the reference splits them.
-#define F64_Q 64  // per-warp ring of queued pairs (power of two, >= 63)
+// Forces, one warp per cell.  The records of the 27 cells around it (src/force/pair_dpd.cu:
+// 292-403, pair_mdpd.cu:399-521) are staged in shared memory once, cell by cell in a fixed
+// order and each cell's records in index order; the cell's atoms are then taken one after the
+// other, each against the staged records 32 at a time, and the pairs inside the largest cutoff
+// are queued in ballot order.  Whenever 32 are queued every lane evaluates one (the Saru random
+// force, the FP64 force) and a segmented tree over the lanes sums the pairs of each atom, so
+// the queue is shared by the cell's atoms and the sums repeat bit for bit.  Four lanes per atom
+// share out its bonds (src/force/bond_harmonic.cu:208-268; FENE + WCA as the FP32 engine) and
+// harmonic angles (src/force/angle_harmonic.cu:187-270).  On logged steps the atom's share of
+// the energies and of the virial: half of each pair and bond, a third of each angle, as the
+// reference splits them.
+// Issue and latency bound it (54% of the issue slots, 20 to 28 warps per SM by registers).
+// With a warp per atom every atom found its candidates' cells anew and its 12.6 pairs ran on
+// 32 lanes (1048 warp instructions an atom); a whole step of the 192k melt went from 279 to
+// 206 us, of the 648k melt from 924 to 658, of 24k from 63 to 51.  7 blocks per SM; 8 and 10
+// spill (211 and 227 us at 192k).  Velocities beside the records instead of by atom index: no
+// gain (231 against 228 us) for twice the cell memory.
+#define F64_Q 64      // queued pairs (power of two, >= 63)
+#define F64_TILE 128  // staged records (27 cells of about 3 atoms, more in several rounds)
+#define F64_HOME 8    // atoms of the cell taken per round
+#define F64_WARPS 4   // warps per block
 
 template <bool LOG>
-__device__ __forceinline__ void f64_pairs(const F64Args& a, int i, int ti, double rho_i, uint32_t step,
-                                          const double4* qd, const int* qj, uint32_t head, int cnt, int lane,
-                                          double& fx, double& fy, double& fz, double& pe, double (&vir)[6])
+struct F64Warp {
+    static constexpr int NV = LOG ? 10 : 3;  // fx fy fz [pe, virial]
+    double4 rec[F64_TILE];                   // staged: position (the image next to the cell), index
+    double4 hx[F64_HOME], hv[F64_HOME];      // the round's atoms: position, index; velocity, type
+    double acc[F64_HOME][NV];
+    double rho[F64_HOME];
+    unsigned short q[F64_Q];                 // queued: staged record * F64_HOME + home atom
+};
+
+// the first cnt queued pairs from `head`, one per lane, added to their atoms' sums
+template <bool LOG>
+__device__ __forceinline__ void f64_pairs(const F64Args& a, uint32_t step, F64Warp<LOG>& w, uint32_t head, int cnt,
+                                          int lane)
 {
-    if (lane >= cnt) return;
-    const uint32_t e = (head + lane) & (F64_Q - 1);
-    const double4 d = qd[e];
-    const int j = qj[e];
-    const double dx = d.x, dy = d.y, dz = d.z, r2 = d.w;
-    const double* c = a.coeff + NC * tri(ti, a.type[j], a.ntypes);
-    if (!(r2 <= c[8])) return;
-    const double A = c[0], B = c[1], gamma = c[2], rc = c[3], rd = c[4], sigma = c[5];
-    // 1/r by rsqrt and r/rc as r * (1/rc): within an ulp of the divisions
-    const double rinv = rsqrt(r2);
-    const double r = r2 * rinv;
-    if (r < 1.0e-10) return;
-    const double dot = dx * (a.v[3 * i] - a.v[3 * j]) + dy * (a.v[3 * i + 1] - a.v[3 * j + 1]) +
-                       dz * (a.v[3 * i + 2] - a.v[3 * j + 2]);
-    const double wc = 1.0 - r * c[6];
-    const uint32_t t1 = (uint32_t)min(i, j) + 1u, t2 = (uint32_t)max(i, j) + 1u;
-    const double theta = saru_theta_f64(t1, t2, a.seed, step);
-    double fpair, e2;
-    if (a.style == 0) {
-        fpair = A * wc - gamma * wc * wc * dot * rinv + sigma * wc * theta;
-        e2 = 0.5 * A * rc * wc * wc;
-    } else {
-        double wd = 1.0 - r * c[7];
-        if (wd < 0.0) wd = 0.0;
-        const double rs = rho_i + a.rho[j];
-        fpair = A * wc + B * rs * wd - gamma * wc * wc * dot * rinv + sigma * wc * theta;
-        e2 = 0.5 * A * rc * wc * wc + 0.25 * B * rd * rs * wd * wd;
+    constexpr int NV = F64Warp<LOG>::NV;
+    double val[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) val[k] = 0.0;
+    int h = F64_HOME + lane;  // lanes without a pair: segments of their own
+    if (lane < cnt) {
+        const unsigned q = w.q[(head + lane) & (F64_Q - 1)];
+        h = (int)(q & (F64_HOME - 1));
+        const double4 xj = w.rec[q / F64_HOME], xi = w.hx[h], vi = w.hv[h];
+        const int i = rec_index(xi), j = rec_index(xj);
+        const double dvx = vi.x - a.v[3 * j], dvy = vi.y - a.v[3 * j + 1], dvz = vi.z - a.v[3 * j + 2];
+        const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        const double* c = a.coeff + NC * tri(rec_index(vi), a.type[j], a.ntypes);
+        // 1/r by rsqrt and r/rc as r * (1/rc): within an ulp of the divisions
+        const double rinv = rsqrt(r2);
+        const double r = r2 * rinv;
+        if (r2 <= c[8] && !(r < 1.0e-10)) {
+            const double A = c[0], B = c[1], gamma = c[2], rc = c[3], rd = c[4], sigma = c[5];
+            const double dot = dx * dvx + dy * dvy + dz * dvz;
+            const double wc = 1.0 - r * c[6];
+            const uint32_t t1 = (uint32_t)min(i, j) + 1u, t2 = (uint32_t)max(i, j) + 1u;
+            const double theta = saru_theta_f64(t1, t2, a.seed, step);
+            double fpair, e2;
+            if (a.style == 0) {
+                fpair = A * wc - gamma * wc * wc * dot * rinv + sigma * wc * theta;
+                e2 = 0.5 * A * rc * wc * wc;
+            } else {
+                double wd = 1.0 - r * c[7];
+                if (wd < 0.0) wd = 0.0;
+                const double rs = w.rho[h] + a.rho[j];
+                fpair = A * wc + B * rs * wd - gamma * wc * wc * dot * rinv + sigma * wc * theta;
+                e2 = 0.5 * A * rc * wc * wc + 0.25 * B * rd * rs * wd * wd;
+            }
+            fpair *= rinv;
+            const double gx = dx * fpair, gy = dy * fpair, gz = dz * fpair;
+            val[0] = gx;
+            val[1] = gy;
+            val[2] = gz;
+            if (LOG) {
+                val[NV - 7] = 0.5 * e2;
+                val[NV - 6] = 0.5 * dx * gx; val[NV - 5] = 0.5 * dx * gy; val[NV - 4] = 0.5 * dx * gz;
+                val[NV - 3] = 0.5 * dy * gy; val[NV - 2] = 0.5 * dy * gz; val[NV - 1] = 0.5 * dz * gz;
+            }
+        }
     }
-    fpair *= rinv;
-    const double gx = dx * fpair, gy = dy * fpair, gz = dz * fpair;
-    fx += gx;
-    fy += gy;
-    fz += gz;
-    if (LOG) {
-        pe += 0.5 * e2;
-        vir[0] += 0.5 * dx * gx; vir[1] += 0.5 * dx * gy; vir[2] += 0.5 * dx * gz;
-        vir[3] += 0.5 * dy * gy; vir[4] += 0.5 * dy * gz; vir[5] += 0.5 * dz * gz;
+    // the pairs of an atom are on consecutive lanes: a fixed tree within each segment
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const bool same = __shfl_down_sync(0xffffffffu, h, o) == h && lane + o < 32;
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const double t = __shfl_down_sync(0xffffffffu, val[k], o);
+            if (same) val[k] += t;
+        }
     }
+    const int before = __shfl_up_sync(0xffffffffu, h, 1);
+    if (h < F64_HOME && (lane == 0 || before != h))
+#pragma unroll
+        for (int k = 0; k < NV; k++) w.acc[h][k] += val[k];
+    __syncwarp();
 }
 
 template <bool LOG>
-__global__ void __launch_bounds__(256) k64_force(F64Args a, uint32_t step)
+__global__ void __launch_bounds__(F64_WARPS * 32, LOG ? 4 : 7) k64_force(F64Args a, uint32_t step, int ncell)
 {
-    __shared__ double4 s_qd[8][F64_Q];
-    __shared__ int s_qj[8][F64_Q];
-    const int warp = threadIdx.x >> 5;
-    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (i >= a.n) return;  // warp-uniform
-    const int ti = a.type[i];
-    double fx = 0.0, fy = 0.0, fz = 0.0, pe = 0.0, bpe = 0.0, ape = 0.0;
-    double vir[6] = {0, 0, 0, 0, 0, 0};
-    const double rho_i = a.style == 1 ? a.rho[i] : 0.0;
-    const double xi = a.x[3 * i], yi = a.x[3 * i + 1], zi = a.x[3 * i + 2];
-    // lane c < 27: the c-th cell around the atom (c = 9 (ox+1) + 3 (oy+1) + (oz+1); nc >= 3
-    // per dimension, so no cell is visited twice) and its record count
-    int cell = 0, m = 0;
+    extern __shared__ double4 f64_smem[];
+    constexpr int NV = F64Warp<LOG>::NV;
+    F64Warp<LOG>& w = reinterpret_cast<F64Warp<LOG>*>(f64_smem)[threadIdx.x >> 5];
+    const int home = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (home >= ncell) return;  // warp-uniform
+    const int m0 = min(a.cnt[home], a.cap);
+    if (m0 == 0) return;
+    // lane c < 27: the c-th cell around the home cell (c = 9 (ox+1) + 3 (oy+1) + (oz+1); nc >= 3
+    // per dimension, so no cell is visited twice), its record count, and the box lengths that
+    // bring its atoms next to the home cell (-1, 0, 1 per dimension).  A pair inside the cutoff
+    // lies in neighbouring cells, so that image is the nearest one.
+    int cell = 0, m = 0, img = 0;
     if (lane < 27) {
-        const int code = a.ccode[i];
-        int cx = (code & 1023) + lane / 9 - 1, cy = ((code >> 10) & 1023) + (lane / 3) % 3 - 1,
-            cz = (code >> 20) + lane % 3 - 1;
-        cx += cx < 0 ? a.nc[0] : 0; cx -= cx >= a.nc[0] ? a.nc[0] : 0;
-        cy += cy < 0 ? a.nc[1] : 0; cy -= cy >= a.nc[1] ? a.nc[1] : 0;
-        cz += cz < 0 ? a.nc[2] : 0; cz -= cz >= a.nc[2] ? a.nc[2] : 0;
-        cell = (cx * a.nc[1] + cy) * a.nc[2] + cz;
+        int cx = home / (a.nc[1] * a.nc[2]) + lane / 9 - 1, cy = (home / a.nc[2]) % a.nc[1] + (lane / 3) % 3 - 1,
+            cz = home % a.nc[2] + lane % 3 - 1;
+        const int wx = (cx >= a.nc[0]) - (cx < 0), wy = (cy >= a.nc[1]) - (cy < 0), wz = (cz >= a.nc[2]) - (cz < 0);
+        cell = ((cx - wx * a.nc[0]) * a.nc[1] + cy - wy * a.nc[1]) * a.nc[2] + cz - wz * a.nc[2];
+        img = (wx + 1) | (wy + 1) << 2 | (wz + 1) << 4;
         m = min(a.cnt[cell], a.cap);
     }
     int incl = m;
@@ -254,153 +298,189 @@ __global__ void __launch_bounds__(256) k64_force(F64Args a, uint32_t step)
     const int excl = incl - m;
     const int M = __shfl_sync(0xffffffffu, incl, 31);
     const unsigned lt = (1u << lane) - 1u;
-    uint32_t head = 0, tail = 0;
-    for (int cb = 0; cb < M; cb += 32) {
-        const int t = cb + lane;
-        // the candidate's cell: the last of the 27 whose first record is at or before t
-        // (an empty cell shares its start with the next one, which then wins)
-        int c = 0;
+    for (int h0 = 0; h0 < m0; h0 += F64_HOME) {
+        const int nh = min(F64_HOME, m0 - h0);
+        if (lane < nh) {
+            const double4 x = a.crec[(size_t)home * a.cap + h0 + lane];
+            w.hx[lane] = x;
+            const int i = rec_index(x);
+            w.hv[lane] = make_double4(a.v[3 * i], a.v[3 * i + 1], a.v[3 * i + 2], rec_word(a.type[i]));
+            if (a.style == 1) w.rho[lane] = a.rho[i];
 #pragma unroll
-        for (int stp = 16; stp >= 1; stp >>= 1) {
-            const int probe = min(c + stp, 26);
-            const int pstart = __shfl_sync(0xffffffffu, excl, probe);
-            if (c + stp <= 26 && pstart <= t) c += stp;
+            for (int k = 0; k < NV; k++) w.acc[lane][k] = 0.0;
         }
-        const int cc = __shfl_sync(0xffffffffu, cell, c);
-        const int c0 = __shfl_sync(0xffffffffu, excl, c);
-        bool hit = false;
-        double dx = 0.0, dy = 0.0, dz = 0.0, r2 = 0.0;
-        int j = 0;
-        if (t < M) {
-            const double4 rj = a.crec[(size_t)cc * a.cap + (t - c0)];
-            j = (int)rj.w;
-            dx = min_image(xi - rj.x, a.L[0]);
-            dy = min_image(yi - rj.y, a.L[1]);
-            dz = min_image(zi - rj.z, a.L[2]);
-            r2 = dx * dx + dy * dy + dz * dz;
-            hit = j != i && r2 <= a.maxrc2;
-        }
-        const unsigned bm = __ballot_sync(0xffffffffu, hit);
-        if (hit) {
-            const uint32_t e = (tail + __popc(bm & lt)) & (F64_Q - 1);
-            s_qd[warp][e] = make_double4(dx, dy, dz, r2);
-            s_qj[warp][e] = j;
-        }
-        tail += __popc(bm);
-        __syncwarp();
-        if (tail - head >= 32u) {
-            f64_pairs<LOG>(a, i, ti, rho_i, step, s_qd[warp], s_qj[warp], head, 32, lane, fx, fy, fz, pe, vir);
-            head += 32;
+        uint32_t head = 0, tail = 0;
+        for (int tb = 0; tb < M; tb += F64_TILE) {
+            const int nt = min(F64_TILE, M - tb);
+            if (h0 == 0 || M > F64_TILE) {
+                for (int q = lane; q < nt + lane; q += 32) {  // uniform trip count (shuffles)
+                    const int t = tb + q;
+                    // the candidate's cell: the last of the 27 whose first record is at or
+                    // before t (an empty cell shares its start with the next one, which then wins)
+                    int c = 0;
+#pragma unroll
+                    for (int stp = 16; stp >= 1; stp >>= 1) {
+                        const int probe = min(c + stp, 26);
+                        const int pstart = __shfl_sync(0xffffffffu, excl, probe);
+                        if (c + stp <= 26 && pstart <= t) c += stp;
+                    }
+                    const int cc = __shfl_sync(0xffffffffu, cell, c);
+                    const int c0 = __shfl_sync(0xffffffffu, excl, c);
+                    const int im = __shfl_sync(0xffffffffu, img, c);
+                    if (q < nt) {
+                        double4 rj = a.crec[(size_t)cc * a.cap + (t - c0)];
+                        rj.x += (im & 3) == 1 ? 0.0 : ((im & 3) ? a.L[0] : -a.L[0]);
+                        rj.y += ((im >> 2) & 3) == 1 ? 0.0 : (((im >> 2) & 3) ? a.L[1] : -a.L[1]);
+                        rj.z += (im >> 4) == 1 ? 0.0 : ((im >> 4) ? a.L[2] : -a.L[2]);
+                        w.rec[q] = rj;
+                    }
+                }
+            }
             __syncwarp();
-        }
-    }
-    if (tail != head)
-        f64_pairs<LOG>(a, i, ti, rho_i, step, s_qd[warp], s_qj[warp], head, (int)(tail - head), lane, fx, fy, fz,
-                       pe, vir);
-    for (int b = a.bstart[i] + lane; b < a.bstart[i + 1]; b += 32) {
-        const int2 e2 = a.bent[b];
-        const int j = e2.x;
-        const double dx = min_image(a.x[3 * i] - a.x[3 * j], a.L[0]);
-        const double dy = min_image(a.x[3 * i + 1] - a.x[3 * j + 1], a.L[1]);
-        const double dz = min_image(a.x[3 * i + 2] - a.x[3 * j + 2], a.L[2]);
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        const double r = sqrt(r2);
-        const double* bc = a.bondc + 4 * (e2.y - 1);
-        double fbond = 0.0, e = 0.0;
-        if (a.bond_style == 1) {
-            fbond = r > 0.0 ? -2.0 * bc[0] * (r - bc[1]) / r : 0.0;
-            e = bc[0] * (r - bc[1]) * (r - bc[1]);
-        } else if (a.bond_style == 2) {
-            const double K = bc[0], R0 = bc[1], eps = bc[2], sg = bc[3];
-            double rr = r2 / (R0 * R0);
-            if (rr >= 1.0) {
-                atomicOr(a.status, F64_FENE);
-                rr = 0.999;
+            for (int h = 0; h < nh; h++) {
+                const double4 xi = w.hx[h];
+                const int i0 = rec_index(xi);
+                for (int q = lane; q < nt + lane; q += 32) {
+                    bool hit = false;
+                    if (q < nt) {
+                        const double4 rj = w.rec[q];
+                        const double dx = xi.x - rj.x, dy = xi.y - rj.y, dz = xi.z - rj.z;
+                        hit = rec_index(rj) != i0 && dx * dx + dy * dy + dz * dz <= a.maxrc2;
+                    }
+                    const unsigned bm = __ballot_sync(0xffffffffu, hit);
+                    if (hit) w.q[(tail + __popc(bm & lt)) & (F64_Q - 1)] = (unsigned short)(q * F64_HOME + h);
+                    tail += __popc(bm);
+                    if (tail - head >= 32u) {
+                        __syncwarp();
+                        f64_pairs<LOG>(a, step, w, head, 32, lane);
+                        head += 32;
+                    }
+                }
             }
-            fbond = -K / (1.0 - rr);
-            e = -0.5 * K * R0 * R0 * log(1.0 - rr);
-            if (eps > 0.0 && r2 < 1.2599210498948731647672106 * sg * sg) {  // 2^(1/3) s^2
-                const double sr2 = sg * sg / r2, sr6 = sr2 * sr2 * sr2;
-                fbond += 48.0 * eps * sr6 * (sr6 - 0.5) / r2;
-                e += 4.0 * eps * sr6 * (sr6 - 1.0) + eps;
+            // the rest of the queue: its atoms come again with the next staged records, and a
+            // chunk's pairs of one atom have to be neighbours
+            __syncwarp();
+            if (tail != head) f64_pairs<LOG>(a, step, w, head, (int)(tail - head), lane);
+            head = tail;
+        }
+        // bonds and angles: lanes 4 h .. 4 h + 3 for the round's atom h
+        static_assert(F64_HOME * 4 == 32, "four lanes per atom of a round");
+        const int h = lane >> 2, sub = lane & 3;
+        double fx = 0.0, fy = 0.0, fz = 0.0, bpe = 0.0, ape = 0.0;
+        double vir[6] = {0, 0, 0, 0, 0, 0};
+        const int i = h < nh ? rec_index(w.hx[h]) : 0;
+        if (h < nh) {
+            for (int b = a.bstart[i] + sub; b < a.bstart[i + 1]; b += 4) {
+                const int2 e2 = a.bent[b];
+                const int j = e2.x;
+                const double dx = min_image(a.x[3 * i] - a.x[3 * j], a.L[0]);
+                const double dy = min_image(a.x[3 * i + 1] - a.x[3 * j + 1], a.L[1]);
+                const double dz = min_image(a.x[3 * i + 2] - a.x[3 * j + 2], a.L[2]);
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                const double r = sqrt(r2);
+                const double* bc = a.bondc + 4 * (e2.y - 1);
+                double fbond = 0.0, e = 0.0;
+                if (a.bond_style == 1) {
+                    fbond = r > 0.0 ? -2.0 * bc[0] * (r - bc[1]) / r : 0.0;
+                    e = bc[0] * (r - bc[1]) * (r - bc[1]);
+                } else if (a.bond_style == 2) {
+                    const double K = bc[0], R0 = bc[1], eps = bc[2], sg = bc[3];
+                    double rr = r2 / (R0 * R0);
+                    if (rr >= 1.0) {
+                        atomicOr(a.status, F64_FENE);
+                        rr = 0.999;
+                    }
+                    fbond = -K / (1.0 - rr);
+                    e = -0.5 * K * R0 * R0 * log(1.0 - rr);
+                    if (eps > 0.0 && r2 < 1.2599210498948731647672106 * sg * sg) {  // 2^(1/3) s^2
+                        const double sr2 = sg * sg / r2, sr6 = sr2 * sr2 * sr2;
+                        fbond += 48.0 * eps * sr6 * (sr6 - 0.5) / r2;
+                        e += 4.0 * eps * sr6 * (sr6 - 1.0) + eps;
+                    }
+                }
+                const double gx = dx * fbond, gy = dy * fbond, gz = dz * fbond;
+                fx += gx;
+                fy += gy;
+                fz += gz;
+                if (LOG) {
+                    bpe += 0.5 * e;
+                    vir[0] += 0.5 * dx * gx; vir[1] += 0.5 * dx * gy; vir[2] += 0.5 * dx * gz;
+                    vir[3] += 0.5 * dy * gy; vir[4] += 0.5 * dy * gz; vir[5] += 0.5 * dz * gz;
+                }
+            }
+            for (int t = a.astart[i] + sub; t < a.astart[i + 1]; t += 4) {
+                const int4 an = a.aent[t];
+                double d1[3], d2[3];
+        #pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    d1[c] = min_image(a.x[3 * an.x + c] - a.x[3 * an.y + c], a.L[c]);
+                    d2[c] = min_image(a.x[3 * an.z + c] - a.x[3 * an.y + c], a.L[c]);
+                }
+                const double rsq1 = d1[0] * d1[0] + d1[1] * d1[1] + d1[2] * d1[2];
+                const double rsq2 = d2[0] * d2[0] + d2[1] * d2[1] + d2[2] * d2[2];
+                const double r1 = sqrt(rsq1), r2 = sqrt(rsq2);
+                double c = (d1[0] * d2[0] + d1[1] * d2[1] + d1[2] * d2[2]) / (r1 * r2);
+                c = fmin(fmax(c, -1.0), 1.0);
+                double s = sqrt(1.0 - c * c);
+                if (s < 0.001) s = 0.001;
+                const double kk = a.anglec[2 * (an.w - 1)];
+                const double theta0 = a.anglec[2 * (an.w - 1) + 1] * (3.14159265358979323846 / 180.0);
+                const double dth = acos(c) - theta0;
+                const double aa = -2.0 * kk * dth / s;
+                const double a11 = aa * c / rsq1, a12 = -aa / (r1 * r2), a22 = aa * c / rsq2;
+                double fi[3], fk[3];
+        #pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    fi[q] = a11 * d1[q] + a12 * d2[q];
+                    fk[q] = a22 * d2[q] + a12 * d1[q];
+                }
+                if (i == an.x) {
+                    fx += fi[0]; fy += fi[1]; fz += fi[2];
+                } else if (i == an.z) {
+                    fx += fk[0]; fy += fk[1]; fz += fk[2];
+                } else {
+                    fx -= fi[0] + fk[0]; fy -= fi[1] + fk[1]; fz -= fi[2] + fk[2];
+                }
+                if (LOG) {
+                    const double third = 1.0 / 3.0;
+                    ape += third * kk * dth * dth;
+                    vir[0] += third * (d1[0] * fi[0] + d2[0] * fk[0]);
+                    vir[1] += third * (d1[0] * fi[1] + d2[0] * fk[1]);
+                    vir[2] += third * (d1[0] * fi[2] + d2[0] * fk[2]);
+                    vir[3] += third * (d1[1] * fi[1] + d2[1] * fk[1]);
+                    vir[4] += third * (d1[1] * fi[2] + d2[1] * fk[2]);
+                    vir[5] += third * (d1[2] * fi[2] + d2[2] * fk[2]);
+                }
             }
         }
-        const double gx = dx * fbond, gy = dy * fbond, gz = dz * fbond;
-        fx += gx;
-        fy += gy;
-        fz += gz;
+        auto sum4 = [](double v) {
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            return v;
+        };
+        fx = sum4(fx);
+        fy = sum4(fy);
+        fz = sum4(fz);
         if (LOG) {
-            bpe += 0.5 * e;
-            vir[0] += 0.5 * dx * gx; vir[1] += 0.5 * dx * gy; vir[2] += 0.5 * dx * gz;
-            vir[3] += 0.5 * dy * gy; vir[4] += 0.5 * dy * gz; vir[5] += 0.5 * dz * gz;
-        }
-    }
-    for (int t = a.astart[i] + lane; t < a.astart[i + 1]; t += 32) {
-        const int4 an = a.aent[t];
-        double d1[3], d2[3];
+            bpe = sum4(bpe);
+            ape = sum4(ape);
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            d1[c] = min_image(a.x[3 * an.x + c] - a.x[3 * an.y + c], a.L[c]);
-            d2[c] = min_image(a.x[3 * an.z + c] - a.x[3 * an.y + c], a.L[c]);
+            for (int k = 0; k < 6; k++) vir[k] = sum4(vir[k]);
         }
-        const double rsq1 = d1[0] * d1[0] + d1[1] * d1[1] + d1[2] * d1[2];
-        const double rsq2 = d2[0] * d2[0] + d2[1] * d2[1] + d2[2] * d2[2];
-        const double r1 = sqrt(rsq1), r2 = sqrt(rsq2);
-        double c = (d1[0] * d2[0] + d1[1] * d2[1] + d1[2] * d2[2]) / (r1 * r2);
-        c = fmin(fmax(c, -1.0), 1.0);
-        double s = sqrt(1.0 - c * c);
-        if (s < 0.001) s = 0.001;
-        const double kk = a.anglec[2 * (an.w - 1)];
-        const double theta0 = a.anglec[2 * (an.w - 1) + 1] * (3.14159265358979323846 / 180.0);
-        const double dth = acos(c) - theta0;
-        const double aa = -2.0 * kk * dth / s;
-        const double a11 = aa * c / rsq1, a12 = -aa / (r1 * r2), a22 = aa * c / rsq2;
-        double fi[3], fk[3];
+        if (h < nh && sub == 0) {
+            a.f[3 * i] = w.acc[h][0] + fx;
+            a.f[3 * i + 1] = w.acc[h][1] + fy;
+            a.f[3 * i + 2] = w.acc[h][2] + fz;
+            if (LOG) {
+                double* q = a.q + (size_t)NQ * i;
+                q[0] = w.acc[h][NV - 7];
+                q[1] = bpe;
+                q[2] = ape;
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
-            fi[q] = a11 * d1[q] + a12 * d2[q];
-            fk[q] = a22 * d2[q] + a12 * d1[q];
+                for (int k = 0; k < 6; k++) q[3 + k] = w.acc[h][NV - 6 + k] + vir[k];
+            }
         }
-        if (i == an.x) {
-            fx += fi[0]; fy += fi[1]; fz += fi[2];
-        } else if (i == an.z) {
-            fx += fk[0]; fy += fk[1]; fz += fk[2];
-        } else {
-            fx -= fi[0] + fk[0]; fy -= fi[1] + fk[1]; fz -= fi[2] + fk[2];
-        }
-        if (LOG) {
-            const double third = 1.0 / 3.0;
-            ape += third * kk * dth * dth;
-            vir[0] += third * (d1[0] * fi[0] + d2[0] * fk[0]);
-            vir[1] += third * (d1[0] * fi[1] + d2[0] * fk[1]);
-            vir[2] += third * (d1[0] * fi[2] + d2[0] * fk[2]);
-            vir[3] += third * (d1[1] * fi[1] + d2[1] * fk[1]);
-            vir[4] += third * (d1[1] * fi[2] + d2[1] * fk[2]);
-            vir[5] += third * (d1[2] * fi[2] + d2[2] * fk[2]);
-        }
-    }
-    fx = warp_sum(fx);
-    fy = warp_sum(fy);
-    fz = warp_sum(fz);
-    if (lane == 0) {
-        a.f[3 * i] = fx;
-        a.f[3 * i + 1] = fy;
-        a.f[3 * i + 2] = fz;
-    }
-    if (LOG) {
-        pe = warp_sum(pe);
-        bpe = warp_sum(bpe);
-        ape = warp_sum(ape);
-#pragma unroll
-        for (int k = 0; k < 6; k++) vir[k] = warp_sum(vir[k]);
-        if (lane == 0) {
-            double* q = a.q + (size_t)NQ * i;
-            q[0] = pe;
-            q[1] = bpe;
-            q[2] = ape;
-#pragma unroll
-            for (int k = 0; k < 6; k++) q[3 + k] = vir[k];
-        }
+        __syncwarp();  // the round's atoms are read before the next round's
     }
 }
 
@@ -514,7 +594,7 @@ int EngineF64::fail(cudaError_t e, const char* what)
 
 EngineF64::~EngineF64()
 {
-    void* ptrs[] = {x_, v_, f_, rho_, q_, part_, sums_, img_, type_, cnt_, ccode_, crec_, status_,
+    void* ptrs[] = {x_, v_, f_, rho_, q_, part_, sums_, img_, type_, cnt_, ccode_, craw_, crec_, status_,
                     bstart_, astart_, bent_, aent_, tab_};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -679,6 +759,7 @@ int EngineF64::init(Replica&& rep)
     F64_CK(dalloc64(&type_, n, bytes_));
     F64_CK(dalloc64(&cnt_, (size_t)ncell_, bytes_));
     F64_CK(dalloc64(&ccode_, n, bytes_));
+    F64_CK(dalloc64(&craw_, (size_t)ncell_ * cap_, bytes_));
     F64_CK(dalloc64(&crec_, (size_t)ncell_ * cap_, bytes_));
     F64_CK(dalloc64(&status_, 1, bytes_));
     F64_CK(dalloc64(&bstart_, n + 1, bytes_));
@@ -767,16 +848,17 @@ int EngineF64::eval_forces(uint32_t step, bool log)
     a.bondc = tab_ + NC * ntri + nt;
     a.anglec = tab_ + NC * ntri + nt + 4 * nbt;
     a.x = x_; a.v = v_; a.f = f_; a.rho = rho_; a.q = q_;
-    a.img = img_; a.type = type_; a.cnt = cnt_; a.crec = crec_; a.status = status_; a.ccode = ccode_;
+    a.img = img_; a.type = type_; a.cnt = cnt_; a.craw = craw_; a.crec = crec_; a.status = status_; a.ccode = ccode_;
     a.bstart = bstart_; a.astart = astart_; a.bent = bent_; a.aent = aent_;
     const int g = (n_ + 255) / 256, gc = (ncell_ + 255) / 256;
     const int gw = (int)(((size_t)n_ * 32 + 255) / 256);  // a warp per atom
     k64_clear<<<gc, 256, 0, stream_>>>(cnt_, ncell_);
     k64_bin<<<g, 256, 0, stream_>>>(a);
-    k64_sort_cells<<<gc, 256, 0, stream_>>>(a, ncell_);
+    k64_sort_cells<<<(int)(((size_t)ncell_ * 8 + 255) / 256), 256, 0, stream_>>>(a, ncell_);
     if (a.style == 1) k64_density<<<gw, 256, 0, stream_>>>(a);
-    if (log) k64_force<true><<<gw, 256, 0, stream_>>>(a, step);
-    else k64_force<false><<<gw, 256, 0, stream_>>>(a, step);
+    const int gf = (ncell_ + F64_WARPS - 1) / F64_WARPS, tf = F64_WARPS * 32;  // a warp per cell
+    if (log) k64_force<true><<<gf, tf, F64_WARPS * sizeof(F64Warp<true>), stream_>>>(a, step, ncell_);
+    else k64_force<false><<<gf, tf, F64_WARPS * sizeof(F64Warp<false>), stream_>>>(a, step, ncell_);
     F64_CK(cudaGetLastError());
     return DPD_OK;
 }

@@ -57,7 +57,8 @@ private:
     double* sums_ = nullptr;     // reduced thermo sums
     int *img_ = nullptr, *type_ = nullptr, *cnt_ = nullptr, *ccode_ = nullptr;
     int* status_ = nullptr;
-    double4* crec_ = nullptr;    // cell records (position, atom index), cap_ per cell
+    int* craw_ = nullptr;        // atom indices appended to each cell, cap_ per cell
+    double4* crec_ = nullptr;    // cell records in index order (position, atom index), cap_ per cell
     int *bstart_ = nullptr, *astart_ = nullptr;
     int2* bent_ = nullptr;       // bond partner index, bond type (1-based)
     int4* aent_ = nullptr;       // angle atoms i, j (apex), k as indices, angle type (1-based)
