@@ -35,7 +35,9 @@ struct F64Args {
     double lo[3], L[3], w[3], dt, maxrc2;
     const double *coeff, *mass, *bondc, *anglec;
     double *x, *v, *f, *rho, *q;
+    double *xn, *vn;  // the next step's positions and velocities (fused step)
     int *img, *type, *cnt, *status;
+    int* cnt_next;    // cell counts of the next binning, cleared by this step's sort
     int* craw;      // atom indices appended to each cell, cap per cell
     double4* crec;  // cell records in index order: position and atom index (rec_index)
     int* ccode;  // each atom's cell as cx | cy << 10 | cz << 20, written by the binning
@@ -62,6 +64,10 @@ __device__ __forceinline__ int tri(int ti, int tj, int nt)
     return ((a - 1) * nt - (a - 1) * (a - 2) / 2 + b - a + 1) - 1;
 }
 
+// Kernels launched with programmatic dependent launch wait here until their predecessor's
+// memory is visible; without a programmatic predecessor the wait returns at once.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ int cell_of(const F64Args& a, const double* p, int c[3])
 {
 #pragma unroll
@@ -72,35 +78,35 @@ __device__ __forceinline__ int cell_of(const F64Args& a, const double* p, int c[
     return (c[0] * a.nc[1] + c[1]) * a.nc[2] + c[2];
 }
 
-__global__ void k64_clear(int* p, int n)
+// an atom into its cell (appended in the order the atomics draw)
+__device__ __forceinline__ void bin_atom(const F64Args& a, int i, const double* x, int* cnt)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = 0;
-}
-
-// atoms into their cells (appended in the order the atomics draw)
-__global__ void k64_bin(F64Args a)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
     int c[3];
-    const int cell = cell_of(a, a.x + 3 * i, c);
+    const int cell = cell_of(a, x, c);
     a.ccode[i] = c[0] | (c[1] << 10) | (c[2] << 20);
-    const int k = atomicAdd(a.cnt + cell, 1);
+    const int k = atomicAdd(cnt + cell, 1);
     if (k < a.cap) a.craw[(size_t)cell * a.cap + k] = i;
     else atomicOr(a.status, F64_CELL_OVERFLOW);
 }
 
+__global__ void k64_bin(F64Args a)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < a.n) bin_atom(a, i, a.x + 3 * i, a.cnt);
+}
+
 // each cell's records in atom-index order, so the pair sums run in a fixed order: 8 lanes per
 // cell rank its indices (a record's place is the number of smaller indices) and gather the
-// records
+// records; the counts that the next binning starts from are cleared
 __global__ void __launch_bounds__(256) k64_sort_cells(F64Args a, int ncell)
 {
+    dep_wait();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = g >> 3;
     if (c >= ncell) return;
     const int* raw = a.craw + (size_t)c * a.cap;
     const int m = min(a.cnt[c], a.cap);
+    if ((g & 7) == 0) a.cnt_next[c] = 0;
     for (int k = g & 7; k < m; k += 8) {
         const int i = raw[k];
         int place = 0;
@@ -150,6 +156,7 @@ __device__ __forceinline__ double warp_sum(double v)
 // atom, lane c takes the c-th of the 27 cells.
 __global__ void __launch_bounds__(256) k64_density(F64Args a)
 {
+    dep_wait();
     const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (i >= a.n) return;  // warp-uniform
     const int ti = a.type[i];
@@ -166,6 +173,35 @@ __global__ void __launch_bounds__(256) k64_density(F64Args a)
     if (lane == 0) a.rho[i] = rho;
 }
 
+__device__ __forceinline__ bool integrated(const F64Args& a, int t)
+{
+    return !a.integ_mask || ((a.integ_mask >> (t - 1)) & 1u);
+}
+
+// a drifted coordinate with the reference's wrap (a while loop moving whole box lengths and
+// counting images); a non-finite coordinate, or one more than 4 box lengths away after a
+// step, is an error
+__device__ __forceinline__ double wrap_coord(const F64Args& a, double p, int d, int* img)
+{
+    const double hi = a.lo[d] + a.L[d];
+    if (!isfinite(p)) {
+        atomicOr(a.status, F64_NONFINITE);
+        p = a.lo[d];
+    }
+    int guard = 0;
+    while ((p >= hi || p < a.lo[d]) && guard < 4) {
+        const int k = (p >= hi) - (p < a.lo[d]);
+        p -= a.L[d] * k;
+        *img += k;
+        guard++;
+    }
+    if (p >= hi || p < a.lo[d]) {
+        atomicOr(a.status, F64_FAR);
+        p = a.lo[d];
+    }
+    return p;
+}
+
 // Forces, one warp per cell.  The records of the 27 cells around it (src/force/pair_dpd.cu:
 // 292-403, pair_mdpd.cu:399-521) are staged in shared memory once, cell by cell in a fixed
 // order and each cell's records in index order; the cell's atoms are then taken one after the
@@ -174,7 +210,12 @@ __global__ void __launch_bounds__(256) k64_density(F64Args a)
 // force, the FP64 force) and a segmented tree over the lanes sums the pairs of each atom, so
 // the queue is shared by the cell's atoms and the sums repeat bit for bit.  Four lanes per atom
 // share out its bonds (src/force/bond_harmonic.cu:208-268; FENE + WCA as the FP32 engine) and
-// harmonic angles (src/force/angle_harmonic.cu:187-270).  On logged steps the atom's share of
+// harmonic angles (src/force/angle_harmonic.cu:187-270).  STEP: the warp holds its atoms' whole
+// forces, so it also takes them through the final half kick, the next step's initial half kick
+// and drift, and appends them to their next cells (positions and velocities into the other
+// buffers, which no warp of this launch reads); a step without thermo is then this kernel and
+// the sort in place of six (3000 atoms 34 -> 16 us, 24000 51 -> 34, 192000 206 -> 192, 648000
+// 658 either way).  On logged steps the atom's share of
 // the energies and of the virial: half of each pair and bond, a third of each angle, as the
 // reference splits them.
 // Issue and latency bound it (54% of the issue slots, 20 to 28 warps per SM by registers).
@@ -266,9 +307,10 @@ __device__ __forceinline__ void f64_pairs(const F64Args& a, uint32_t step, F64Wa
     __syncwarp();
 }
 
-template <bool LOG>
+template <bool LOG, bool STEP>
 __global__ void __launch_bounds__(F64_WARPS * 32, LOG ? 4 : 7) k64_force(F64Args a, uint32_t step, int ncell)
 {
+    dep_wait();
     extern __shared__ double4 f64_smem[];
     constexpr int NV = F64Warp<LOG>::NV;
     F64Warp<LOG>& w = reinterpret_cast<F64Warp<LOG>*>(f64_smem)[threadIdx.x >> 5];
@@ -467,10 +509,33 @@ __global__ void __launch_bounds__(F64_WARPS * 32, LOG ? 4 : 7) k64_force(F64Args
 #pragma unroll
             for (int k = 0; k < 6; k++) vir[k] = sum4(vir[k]);
         }
+        double p = 0.0;
+        if (h < nh && sub < 3) {  // a lane per component
+            const double f = w.acc[h][sub] + (sub == 0 ? fx : (sub == 1 ? fy : fz));
+            a.f[3 * i + sub] = f;
+            if (STEP) {
+                const double4 xi = w.hx[h], vi = w.hv[h];
+                double v = sub == 0 ? vi.x : (sub == 1 ? vi.y : vi.z);
+                p = sub == 0 ? xi.x : (sub == 1 ? xi.y : xi.z);
+                const int t = rec_index(vi);
+                if (integrated(a, t)) {
+                    const double dtm = 0.5 * a.dt / a.mass[t - 1];
+                    v += dtm * f;
+                    v += dtm * f;
+                    p = wrap_coord(a, p + a.dt * v, sub, a.img + 3 * i + sub);
+                }
+                a.vn[3 * i + sub] = v;
+                a.xn[3 * i + sub] = p;
+            }
+        }
+        if (STEP) {
+            const double py = __shfl_sync(0xffffffffu, p, (lane & ~3) + 1), pz = __shfl_sync(0xffffffffu, p, (lane & ~3) + 2);
+            if (h < nh && sub == 0) {
+                const double at[3] = {p, py, pz};
+                bin_atom(a, i, at, a.cnt_next);
+            }
+        }
         if (h < nh && sub == 0) {
-            a.f[3 * i] = w.acc[h][0] + fx;
-            a.f[3 * i + 1] = w.acc[h][1] + fy;
-            a.f[3 * i + 2] = w.acc[h][2] + fz;
             if (LOG) {
                 double* q = a.q + (size_t)NQ * i;
                 q[0] = w.acc[h][NV - 7];
@@ -484,14 +549,7 @@ __global__ void __launch_bounds__(F64_WARPS * 32, LOG ? 4 : 7) k64_force(F64Args
     }
 }
 
-__device__ __forceinline__ bool integrated(const F64Args& a, int t)
-{
-    return !a.integ_mask || ((a.integ_mask >> (t - 1)) & 1u);
-}
-
-// half kick and drift with the reference's wrap (a while loop moving whole box lengths
-// and counting images); a non-finite coordinate, or one more than 4 box lengths away
-// after a step, is an error
+// half kick and drift
 __global__ void k64_initial(F64Args a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -502,24 +560,7 @@ __global__ void k64_initial(F64Args a)
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         a.v[3 * i + d] += dtm * a.f[3 * i + d];
-        double p = a.x[3 * i + d] + a.dt * a.v[3 * i + d];
-        const double hi = a.lo[d] + a.L[d];
-        if (!isfinite(p)) {
-            atomicOr(a.status, F64_NONFINITE);
-            p = a.lo[d];
-        }
-        int guard = 0;
-        while ((p >= hi || p < a.lo[d]) && guard < 4) {
-            const int k = (p >= hi) - (p < a.lo[d]);
-            p -= a.L[d] * k;
-            a.img[3 * i + d] += k;
-            guard++;
-        }
-        if (p >= hi || p < a.lo[d]) {
-            atomicOr(a.status, F64_FAR);
-            p = a.lo[d];
-        }
-        a.x[3 * i + d] = p;
+        a.x[3 * i + d] = wrap_coord(a, a.x[3 * i + d] + a.dt * a.v[3 * i + d], d, a.img + 3 * i + d);
     }
 }
 
@@ -594,7 +635,7 @@ int EngineF64::fail(cudaError_t e, const char* what)
 
 EngineF64::~EngineF64()
 {
-    void* ptrs[] = {x_, v_, f_, rho_, q_, part_, sums_, img_, type_, cnt_, ccode_, craw_, crec_, status_,
+    void* ptrs[] = {x_, v_, xn_, vn_, cnt_next_, f_, rho_, q_, part_, sums_, img_, type_, cnt_, ccode_, craw_, crec_, status_,
                     bstart_, astart_, bent_, aent_, tab_};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -750,6 +791,8 @@ int EngineF64::init(Replica&& rep)
     const size_t n = (size_t)n_;
     F64_CK(dalloc64(&x_, 3 * n, bytes_));
     F64_CK(dalloc64(&v_, 3 * n, bytes_));
+    F64_CK(dalloc64(&xn_, 3 * n, bytes_));
+    F64_CK(dalloc64(&vn_, 3 * n, bytes_));
     F64_CK(dalloc64(&f_, 3 * n, bytes_));
     F64_CK(dalloc64(&rho_, n, bytes_));
     F64_CK(dalloc64(&q_, (size_t)NQ * n, bytes_));
@@ -758,6 +801,7 @@ int EngineF64::init(Replica&& rep)
     F64_CK(dalloc64(&img_, 3 * n, bytes_));
     F64_CK(dalloc64(&type_, n, bytes_));
     F64_CK(dalloc64(&cnt_, (size_t)ncell_, bytes_));
+    F64_CK(dalloc64(&cnt_next_, (size_t)ncell_, bytes_));
     F64_CK(dalloc64(&ccode_, n, bytes_));
     F64_CK(dalloc64(&craw_, (size_t)ncell_ * cap_, bytes_));
     F64_CK(dalloc64(&crec_, (size_t)ncell_ * cap_, bytes_));
@@ -839,7 +883,27 @@ static F64Args make_args(const Replica& R, int n, const int nc[3], const double 
     return a;
 }
 
-int EngineF64::eval_forces(uint32_t step, bool log)
+// the launch may overlap the tail of its predecessor (the kernel starts with dep_wait)
+template <typename... KArgs, typename... Args>
+static void launch_dep(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+// The forces of a step from the current positions and velocities.  binned: the previous step
+// has put the atoms into their cells; advance: the force pass also takes them to the next
+// step's positions and cells (steps without thermo), and the buffers change places.
+int EngineF64::eval_forces(uint32_t step, bool log, bool binned, bool advance)
 {
     F64Args a = make_args(R_, n_, nc_, L_, cap_);
     const int nt = R_.sys.n_atomtypes, ntri = nt * (nt + 1) / 2, nbt = std::max(R_.sys.n_bondtypes, 1);
@@ -847,18 +911,25 @@ int EngineF64::eval_forces(uint32_t step, bool log)
     a.mass = tab_ + NC * ntri;
     a.bondc = tab_ + NC * ntri + nt;
     a.anglec = tab_ + NC * ntri + nt + 4 * nbt;
-    a.x = x_; a.v = v_; a.f = f_; a.rho = rho_; a.q = q_;
-    a.img = img_; a.type = type_; a.cnt = cnt_; a.craw = craw_; a.crec = crec_; a.status = status_; a.ccode = ccode_;
+    a.x = x_; a.v = v_; a.f = f_; a.rho = rho_; a.q = q_; a.xn = xn_; a.vn = vn_;
+    a.img = img_; a.type = type_; a.cnt = cnt_; a.cnt_next = cnt_next_; a.craw = craw_; a.crec = crec_;
+    a.status = status_; a.ccode = ccode_;
     a.bstart = bstart_; a.astart = astart_; a.bent = bent_; a.aent = aent_;
-    const int g = (n_ + 255) / 256, gc = (ncell_ + 255) / 256;
     const int gw = (int)(((size_t)n_ * 32 + 255) / 256);  // a warp per atom
-    k64_clear<<<gc, 256, 0, stream_>>>(cnt_, ncell_);
-    k64_bin<<<g, 256, 0, stream_>>>(a);
-    k64_sort_cells<<<(int)(((size_t)ncell_ * 8 + 255) / 256), 256, 0, stream_>>>(a, ncell_);
-    if (a.style == 1) k64_density<<<gw, 256, 0, stream_>>>(a);
+    if (!binned) k64_bin<<<(n_ + 255) / 256, 256, 0, stream_>>>(a);
+    launch_dep(k64_sort_cells, (int)(((size_t)ncell_ * 8 + 255) / 256), 256, 0, stream_, a, ncell_);
+    if (a.style == 1) launch_dep(k64_density, gw, 256, 0, stream_, a);
     const int gf = (ncell_ + F64_WARPS - 1) / F64_WARPS, tf = F64_WARPS * 32;  // a warp per cell
-    if (log) k64_force<true><<<gf, tf, F64_WARPS * sizeof(F64Warp<true>), stream_>>>(a, step, ncell_);
-    else k64_force<false><<<gf, tf, F64_WARPS * sizeof(F64Warp<false>), stream_>>>(a, step, ncell_);
+    if (log) launch_dep(k64_force<true, false>, gf, tf, F64_WARPS * sizeof(F64Warp<true>), stream_, a, step, ncell_);
+    else if (!advance)
+        launch_dep(k64_force<false, false>, gf, tf, F64_WARPS * sizeof(F64Warp<false>), stream_, a, step, ncell_);
+    else {
+        launch_dep(k64_force<false, true>, gf, tf, F64_WARPS * sizeof(F64Warp<false>), stream_, a, step, ncell_);
+        std::swap(x_, xn_);
+        std::swap(v_, vn_);
+    }
+    // the sort has cleared the other counts: the next binning fills them
+    std::swap(cnt_, cnt_next_);
     F64_CK(cudaGetLastError());
     return DPD_OK;
 }
@@ -921,26 +992,32 @@ int EngineF64::run(uint32_t nsteps)
     F64Args a = make_args(R_, n_, nc_, L_, cap_);
     const int nt = R_.sys.n_atomtypes, ntri = nt * (nt + 1) / 2;
     a.mass = tab_ + NC * ntri;
-    a.x = x_; a.v = v_; a.f = f_; a.img = img_; a.type = type_; a.status = status_;
+    a.f = f_; a.img = img_; a.type = type_; a.status = status_;
     const int g = (n_ + 255) / 256;
     const uint32_t log_f = R_.in.log_f;
     int e;
     if (zero_pending_) {
         const uint32_t s0 = next_step_;
         const bool log = s0 % log_f == 0;
-        if ((e = eval_forces(s0, log))) return e;
+        if ((e = eval_forces(s0, log, false, false))) return e;
         if ((e = check_status())) return e;
         if (log && (e = log_row(s0))) return e;
         zero_pending_ = false;
         next_step_ = s0 + 1;
     }
+    bool binned = false;  // the previous step's force pass has already drifted and binned the atoms
     for (uint32_t k = 0; k < nsteps; k++) {
         const uint32_t step = next_step_;
-        const bool log = step % log_f == 0;
-        k64_initial<<<g, 256, 0, stream_>>>(a);
-        if ((e = eval_forces(step, log))) return e;
-        k64_final<<<g, 256, 0, stream_>>>(a);
-        F64_CK(cudaGetLastError());
+        const bool log = step % log_f == 0, advance = !log && k + 1 < nsteps;
+        a.x = x_;
+        a.v = v_;
+        if (!binned) k64_initial<<<g, 256, 0, stream_>>>(a);
+        if ((e = eval_forces(step, log, binned, advance))) return e;
+        binned = advance;
+        if (!advance) {
+            k64_final<<<g, 256, 0, stream_>>>(a);
+            F64_CK(cudaGetLastError());
+        }
         if (log) {
             if ((e = log_row(step))) return e;
             if ((e = check_status())) return e;

@@ -39,7 +39,7 @@ public:
 private:
     int fail(cudaError_t e, const char* what);
     int upload_state(bool pos, bool vel);
-    int eval_forces(uint32_t step, bool log);
+    int eval_forces(uint32_t step, bool log, bool binned, bool advance);
     int check_status();
     int log_row(uint32_t step);
 
@@ -52,11 +52,13 @@ private:
     cudaStream_t stream_ = nullptr;
     // device state, tag order
     double *x_ = nullptr, *v_ = nullptr, *f_ = nullptr, *rho_ = nullptr;
+    double *xn_ = nullptr, *vn_ = nullptr;  // the other buffers of a step that its force pass advances
     double* q_ = nullptr;        // per-atom log terms: pair, bond, angle PE, virial[6]
     double* part_ = nullptr;     // per-block partial sums of the thermo reduction
     double* sums_ = nullptr;     // reduced thermo sums
     int *img_ = nullptr, *type_ = nullptr, *cnt_ = nullptr, *ccode_ = nullptr;
     int* status_ = nullptr;
+    int* cnt_next_ = nullptr;    // cell counts of the next binning
     int* craw_ = nullptr;        // atom indices appended to each cell, cap_ per cell
     double4* crec_ = nullptr;    // cell records in index order (position, atom index), cap_ per cell
     int *bstart_ = nullptr, *astart_ = nullptr;
