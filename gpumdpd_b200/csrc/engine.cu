@@ -289,7 +289,7 @@ int Engine::alloc_and_upload()
     DA(b_.mass, nmass);
     DA(b_.bondc, nbond);
     for (int q = 0; q < 2; q++) {
-        DA(b_.pos[q], P_);
+        DA(b_.pos[q], P_ + 32);  // k_build_lin loads a few slots past the end of a range
         DA(b_.vel[q], P_);
         DA(b_.bonds[q], (size_t)std::max(maxb_, 1) * P_);
     }
@@ -830,20 +830,25 @@ static void launch_pair(int variant, bool bonds, bool filt, int grid, cudaStream
 }
 
 // The list-build chain; every kernel returns at once unless this phase's flag is set.
-void Engine::enqueue_build(cudaStream_t s, bool list, bool wide)
+// linear: the device's cell ranks are those of cell order 0 when it runs.
+void Engine::enqueue_build(cudaStream_t s, bool list, bool wide, bool linear)
 {
     const int nrep = (int)reps_.size();
     BuildArgs ba = build_args(b_, P_, C_, nmax_, maxb_);
     const int gp = (P_ + 255) / 256;
-    const int gc = (C_ + 255) / 256;
+    const int gc = (C_ + 1023) / 1024;
     const int nsb = (C_ + 4095) / 4096;
     pdl_launch(k_bin_count, gp, 256, s, ba);
     if (nsb == 1) {
         pdl_launch(k_scan_blocks<true>, 1, 1024, s, ba);
     } else {
         pdl_launch(k_scan_blocks<false>, nsb, 1024, s, ba);
-        pdl_launch(k_scan_sums, 1, 1024, s, ba, nsb);
-        pdl_launch(k_scan_add, gc, 256, s, ba);
+        if (nsb <= 1024) {
+            pdl_launch(k_scan_add<false>, gc, 1024, s, ba);
+        } else {
+            pdl_launch(k_scan_sums, 1, 1024, s, ba, nsb);
+            pdl_launch(k_scan_add<true>, gc, 1024, s, ba);
+        }
     }
     if (gp <= 148 * 8) {
         pdl_launch(k_permute<true>, gp, 256, s, ba, nrep);
@@ -859,6 +864,7 @@ void Engine::enqueue_build(cudaStream_t s, bool list, bool wide)
         } else if (wide && gp <= 148 * 8) pdl_launch(k_build_wide, (14 * P_ + 255) / 256, 256, s, ba);
         else if (tune_.build_variant == 1) pdl_launch(k_build_nlist_s<6>, gp, 256, s, ba);
         else if (tune_.build_variant == 2) pdl_launch(k_build_nlist_s<8>, gp, 256, s, ba);
+        else if (tune_.build_variant == 5 && linear) pdl_launch(k_build_lin, (P_ + 127) / 128, 128, s, ba);
         else if (tune_.build_variant == 5) pdl_launch(k_build_cols, gp, 256, s, ba);
         else pdl_launch(k_build_nlist, gp, 256, s, ba);
     }
@@ -886,7 +892,8 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     // schedule 6: the DPD list build runs inside the pair kernel
     const bool fused = variant == 6 && !any_mdpd_;
     enqueue_build(s, !fused && !tile,
-                  (tiny && (tune_.build_variant == 0 || tune_.build_variant == 5)) || tune_.build_variant == 3);
+                  (tiny && (tune_.build_variant == 0 || tune_.build_variant == 5)) || tune_.build_variant == 3,
+                  tune_.cell_order == 0);  // a run uploads the ranks of the tuning first
     if (any_mdpd_) pdl_launch(k_density, gp, 256, s, sa);
     if (ev0) cudaEventRecordWithFlags(ev0, s, cudaEventRecordExternal);
     if (tile) {
@@ -1918,7 +1925,8 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
     StepArgs sa = step_args(b_, P_, nmax_, maxb_, 1);
     const int gp = (P_ + 255) / 256;
     k_aos_in<<<(n + 255) / 256, 256, 0, stream_>>>(sa, d_pos, d_vel, d_id, d_type, n, step, aos_built_ ? 0 : 1);
-    enqueue_build(stream_, true, tune_.build_variant == 3);
+    // a changed cell order waits for the next run: until then the device keeps the old ranks
+    enqueue_build(stream_, true, tune_.build_variant == 3, tune_.cell_order == 0 && !ranks_dirty_);
     if (any_mdpd_) k_density<<<gp, 256, 0, stream_>>>(sa);
     const bool peratom = d_pe || d_virial;
     // this entry builds the list itself: schedule 11 (no list) runs as the default 8
