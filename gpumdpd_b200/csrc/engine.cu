@@ -1925,12 +1925,18 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
     StepArgs sa = step_args(b_, P_, nmax_, maxb_, 1);
     const int gp = (P_ + 255) / 256;
     k_aos_in<<<(n + 255) / 256, 256, 0, stream_>>>(sa, d_pos, d_vel, d_id, d_type, n, step, aos_built_ ? 0 : 1);
+    // the launch choices of enqueue_step for small and tiny grids: the list build with a thread
+    // per (slot, stencil cell), the pair pass in one launch
+    const bool small = tune_.launch_mode == 2 || ((tune_.launch_mode == 0 || tune_.launch_mode == 3) && gp <= 148 * 8);
+    const bool tiny = small && gp <= 148 && tune_.launch_mode != 3;
     // a changed cell order waits for the next run: until then the device keeps the old ranks
-    enqueue_build(stream_, true, tune_.build_variant == 3, tune_.cell_order == 0 && !ranks_dirty_);
-    if (any_mdpd_) k_density<<<gp, 256, 0, stream_>>>(sa);
+    enqueue_build(stream_, true, (tiny && (tune_.build_variant == 0 || tune_.build_variant == 5)) || tune_.build_variant == 3,
+                  tune_.cell_order == 0 && !ranks_dirty_);
+    if (any_mdpd_) pdl_launch(k_density, gp, 256, stream_, sa);
     const bool peratom = d_pe || d_virial;
     // this entry builds the list itself: schedule 11 (no list) runs as the default 8
-    const int pv = tune_.pair_variant == 11 ? 8 : tune_.pair_variant;
+    int pv = tune_.pair_variant == 11 ? 8 : tune_.pair_variant;
+    if (pv == 8 && small) pv = 4;
     if (d.style == 0) {
         if (peratom) k_pair_peratom<0><<<gp, 256, 0, stream_>>>(sa, pe_slot_, vir_slot_);
         else launch_pair<0>(pv, false, filt_, gp, stream_, sa);
@@ -1938,8 +1944,7 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
         if (peratom) k_pair_peratom<1><<<gp, 256, 0, stream_>>>(sa, pe_slot_, vir_slot_);
         else launch_pair<1>(pv, false, filt_, gp, stream_, sa);
     }
-    k_aos_out<<<gp, 256, 0, stream_>>>(sa, d_force, d_pe, d_virial, pe_slot_, vir_slot_);
-    k_aos_done<<<1, 1, 0, stream_>>>(b_.build_flag, b_.phase);
+    pdl_launch(k_aos_out, gp, 256, stream_, sa, d_force, d_pe, d_virial, pe_slot_, vir_slot_);
     CK(cudaGetLastError());
     aos_built_ = true;
     return sync_and_check();

@@ -138,11 +138,14 @@ __global__ void __launch_bounds__(256) k_pair_peratom(StepArgs a, float* pe_slot
     atomicAdd(&vir_slot[6 * (size_t)s + 5], v5);
 }
 
-// engine slots -> AoS (index = tag - 1); clears the slot accumulators for the next call
+// engine slots -> AoS (index = tag - 1); clears the slot accumulators and the build flag for
+// the next call
 __global__ void k_aos_out(StepArgs a, float* fout, float* pe_out, float* vir_out, float* pe_slot,
                           float* vir_slot)
 {
+    griddep_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s == 0) a.build_flag[*a.phase & 1] = 0;
     if (s >= a.P) return;
     const RepDesc& d = a.reps[0];
     if (s >= d.p_end) return;
@@ -164,11 +167,6 @@ __global__ void k_aos_out(StepArgs a, float* fout, float* pe_out, float* vir_out
             vir_slot[6 * (size_t)s + c] = 0.0f;
         }
     }
-}
-
-__global__ void k_aos_done(int* build_flag, const uint32_t* phase)
-{
-    build_flag[(*phase) & 1] = 0;
 }
 
 // ---------------------------------------------------------------------------------
