@@ -58,6 +58,7 @@ struct RepDesc {
     float L[3];
     float cut2;     // (global_cut + skin)^2 in float, list predicate
     float rcmax2;   // max over type pairs of rc^2
+    float rdmax2;   // max over type pairs of rd^2 (mDPD density)
     float hskin2;   // (skin/2)^2
     int skin_zero;  // skin == 0: rebuild every nl_f steps unconditionally
     int ntypes;

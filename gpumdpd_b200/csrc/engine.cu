@@ -171,9 +171,14 @@ int Engine::layout()
         tag_base += n;
         const float cutf = (float)cut;
         d.cut2 = cutf * cutf;
-        double rcm = 0;
-        for (auto& c : R.ff.coeff) rcm = std::max(rcm, c[3]);
+        double rcm = 0, rdm = 0;
+        for (auto& c : R.ff.coeff) {
+            rcm = std::max(rcm, c[3]);
+            rdm = std::max(rdm, c[4]);
+        }
         d.rcmax2 = (float)(rcm * rcm);
+        // not below the pairs' own rd^2, which are squared in float
+        d.rdmax2 = (float)rdm * (float)rdm;
         const float hs = (float)(R.in.skin * 0.5);
         d.hskin2 = hs * hs;
         if (d.cut2 > d.rcmax2) filt_ = true;
@@ -311,6 +316,10 @@ int Engine::alloc_and_upload()
     DA(b_.img, ntag);
     DA(b_.ncount, P_);
     DA(b_.nlist, (size_t)P_ * nmax_);
+    if (any_mdpd_) {
+        DA(b_.near_list, (size_t)P_ * nmax_);
+        DA(b_.near_count, P_);
+    }
     DA(b_.blocksum, (C_ + 4095) / 4096 + 1);
     DA(b_.acc, (size_t)nrep * DPD_ACC_SLOTS * DPD_NACC);
     DA(b_.ring, (size_t)nrep * DPD_RING_ROWS * DPD_THERMO_FIELDS);
@@ -894,7 +903,10 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     enqueue_build(s, !fused && !tile,
                   (tiny && (tune_.build_variant == 0 || tune_.build_variant == 5)) || tune_.build_variant == 3,
                   tune_.cell_order == 0);  // a run uploads the ranks of the tuning first
-    if (any_mdpd_) pdl_launch(k_density, gp, 256, s, sa);
+    StepArgs sm = sa;  // mDPD: the force pass takes the density pass's list
+    sm.nlist = b_.near_list;
+    sm.ncount = b_.near_count;
+    if (any_mdpd_) pdl_launch(k_density, gp, 256, s, sa, b_.near_list, b_.near_count);
     if (ev0) cudaEventRecordWithFlags(ev0, s, cudaEventRecordExternal);
     if (tile) {
         const TileArgs ta{b_.tile_rep, b_.tile_code, ntiles_, tile_edge_, tile_smax_, tile_hc_};
@@ -921,7 +933,7 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     } else if (any_dpd_) {
         launch_pair<0>(variant, bonds_, filt_, gp, s, sa);
     }
-    if (any_mdpd_) launch_pair<1>(variant, bonds_, filt_, gp, s, sa);
+    if (any_mdpd_) launch_pair<1>(variant, bonds_, false, gp, s, sm);
     if (ev1) cudaEventRecordWithFlags(ev1, s, cudaEventRecordExternal);
     if (nang_ > 0) pdl_launch(k_angle, (nang_ + 255) / 256, 256, s, sa, angle_tbl_, angle_coef_, angle_wrep_, nang_);
     if (rdf_) pdl_launch(k_rdf, gp, 256, s, sa);
@@ -1296,6 +1308,7 @@ int64_t Engine::estimate_bytes(const std::vector<const Replica*>& reps)
 {
     int64_t P = 0, C = 0, ntag = 0, ncoeff = 0, nmass = 0, nbond = 0, nrdf = 0, nang = 0;
     int64_t nmax = 16, maxb = 0;
+    bool mdpd = false;
     const int64_t nrep = (int64_t)reps.size();
     for (const Replica* R : reps) nang += ((int64_t)(R->sys.angles.size() / 4) + 31) / 32 * 32;
     for (const Replica* R : reps) {
@@ -1304,6 +1317,7 @@ int64_t Engine::estimate_bytes(const std::vector<const Replica*>& reps)
         for (int k = 0; k < 3; k++)
             ncell *= std::max(1, (int)std::floor((R->sys.hi[k] - R->sys.lo[k]) / cut));
         const int64_t n = R->sys.n_atoms;
+        mdpd = mdpd || R->ff.pair_style == 1;
         P += ((n + 31) / 32) * 32;
         C += ncell + 1;
         ntag += n;
@@ -1328,6 +1342,7 @@ int64_t Engine::estimate_bytes(const std::vector<const Replica*>& reps)
     int64_t bytes = nrep * ((int64_t)sizeof(RepDesc) + (int64_t)sizeof(RepState) + 4);
     bytes += (P / 32) * 4 + ncoeff * 16 + nmass * 8 + nbond * 16 + nrdf * 8;
     bytes += P * (2 * (16 + 16 + 16) + 2 * mb * 8 + 16 + 16 + 4 + 4 + 8 + 4 * nmax + mb * 8);
+    if (mdpd) bytes += P * (4 * nmax + 4);  // the near list
     bytes += C * (4 * 5) + ntag * 4 + ((C + 4095) / 4096 + 1) * 4;
     bytes += nrep * ((int64_t)DPD_ACC_SLOTS * DPD_NACC * 8 + (int64_t)DPD_RING_ROWS * DPD_THERMO_FIELDS * 8);
     bytes += nang * 16 + (nang / 32) * 4 + nrep * 32 * 8;  // angle table, warp replicas, coefficients
@@ -1932,7 +1947,10 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
     // a changed cell order waits for the next run: until then the device keeps the old ranks
     enqueue_build(stream_, true, (tiny && (tune_.build_variant == 0 || tune_.build_variant == 5)) || tune_.build_variant == 3,
                   tune_.cell_order == 0 && !ranks_dirty_);
-    if (any_mdpd_) pdl_launch(k_density, gp, 256, stream_, sa);
+    StepArgs sm = sa;
+    sm.nlist = b_.near_list;
+    sm.ncount = b_.near_count;
+    if (any_mdpd_) pdl_launch(k_density, gp, 256, stream_, sa, b_.near_list, b_.near_count);
     const bool peratom = d_pe || d_virial;
     // this entry builds the list itself: schedule 11 (no list) runs as the default 8
     int pv = tune_.pair_variant == 11 ? 8 : tune_.pair_variant;
@@ -1942,7 +1960,7 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
         else launch_pair<0>(pv, false, filt_, gp, stream_, sa);
     } else {
         if (peratom) k_pair_peratom<1><<<gp, 256, 0, stream_>>>(sa, pe_slot_, vir_slot_);
-        else launch_pair<1>(pv, false, filt_, gp, stream_, sa);
+        else launch_pair<1>(pv, false, false, gp, stream_, sm);
     }
     pdl_launch(k_aos_out, gp, 256, stream_, sa, d_force, d_pe, d_virial, pe_slot_, vir_slot_);
     CK(cudaGetLastError());

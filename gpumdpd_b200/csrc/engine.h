@@ -60,6 +60,7 @@ struct DeviceBuffers {
     int *cell_rep = nullptr, *cell_lin = nullptr;
     int *cnt = nullptr, *cstart = nullptr, *skey = nullptr, *srank = nullptr, *tag2idx = nullptr;
     int *ncount = nullptr, *nlist = nullptr, *blocksum = nullptr;
+    int *near_count = nullptr, *near_list = nullptr;  // mDPD: the entries inside the largest cutoff
     unsigned int* ticket = nullptr;  // k_permute's last-block counter
     unsigned int* ticket2 = nullptr; // k_integrate_adv's last-block counter
     double *acc = nullptr, *ring = nullptr;
