@@ -51,6 +51,7 @@ Engine::~Engine()
 {
     dump_close();
     if (graph_) cudaGraphExecDestroy(graph_);
+    if (graph_many_) cudaGraphExecDestroy(graph_many_);
     if (stream_) cudaStreamSynchronize(stream_);
     for (void* p : allocs_) cudaFreeAsync(p, stream_);
     if (stream_) cudaStreamSynchronize(stream_);
@@ -1080,26 +1081,34 @@ int Engine::refresh_list()
     return DPD_OK;
 }
 
-int Engine::build_graph()
+// steps of a graph launch: 24000 particles take 32.1 us a step with 1, 29.2 with 8 (3000: 23.7 and
+// 20.8; 192000: 71.9 and 70.4); making both graphs takes 0.39 ms against 0.14
+#define DPD_GRAPH_STEPS 8
+
+int Engine::capture_steps(int n, cudaGraphExec_t* out)
 {
-    if (graph_) {
-        cudaGraphExecDestroy(graph_);
-        graph_ = nullptr;
-    }
-    {
-        const int e = prepare_tiles();
-        if (e) return e;
+    if (*out) {
+        cudaGraphExecDestroy(*out);
+        *out = nullptr;
     }
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    enqueue_step(stream_, nullptr, nullptr);
+    for (int k = 0; k < n; k++) enqueue_step(stream_, nullptr, nullptr);
     cudaError_t e = cudaStreamEndCapture(stream_, &g);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
-    e = cudaGraphInstantiate(&graph_, g, 0);
+    e = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
-    CK(cudaGraphUpload(graph_, stream_));
+    CK(cudaGraphUpload(*out, stream_));
     return DPD_OK;
+}
+
+int Engine::build_graph()
+{
+    int e = prepare_tiles();
+    if (!e) e = capture_steps(1, &graph_);
+    if (!e) e = capture_steps(DPD_GRAPH_STEPS, &graph_many_);
+    return e;
 }
 
 // set the run target of every replica (absolute step), optionally mark the next
@@ -1141,7 +1150,9 @@ int Engine::run_async(uint32_t nsteps)
         force_build_ = false;
         if (!zero) enqueue_integrate_initial(stream_);
         CK(cudaGetLastError());
-        for (uint32_t k = s; k <= end; k++) CK(cudaGraphLaunch(graph_, stream_));
+        uint32_t left = end - s + 1;
+        for (; left >= DPD_GRAPH_STEPS; left -= DPD_GRAPH_STEPS) CK(cudaGraphLaunch(graph_many_, stream_));
+        for (; left > 0; left--) CK(cudaGraphLaunch(graph_, stream_));
         zero = false;
         // the host's step counter follows each segment, so a failed frame write leaves
         // it where the device stopped

@@ -202,7 +202,10 @@ private:
     DeviceBuffers b_;
     dpd_tuning tune_{};
     cudaStream_t stream_ = nullptr;
-    cudaGraphExec_t graph_ = nullptr;
+    // one timestep, and DPD_GRAPH_STEPS of them as one launch (their kernels overlap as those
+    // within a step do; consecutive graph launches do not)
+    cudaGraphExec_t graph_ = nullptr, graph_many_ = nullptr;
+    int capture_steps(int n, cudaGraphExec_t* out);
     int P_ = 0, C_ = 0, nmax_ = 16, maxb_ = 0;
     bool any_mdpd_ = false, any_dpd_ = false, bonds_ = false, rdf_ = false;
     bool any_spring_ = false, any_eos_ = false;  // some replica has a spring / an rvcm or recenter
