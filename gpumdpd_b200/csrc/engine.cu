@@ -275,6 +275,8 @@ int Engine::init(std::vector<Replica>&& reps, const dpd_tuning* tune)
     return build_graph();
 }
 
+static StepArgs step_args(const DeviceBuffers& b, int P, int nmax, int maxb, int nrep);
+
 int Engine::alloc_and_upload()
 {
     const int nrep = (int)reps_.size();
@@ -544,7 +546,11 @@ int Engine::alloc_and_upload()
         CK(cudaMemcpyAsync(b_.uw0, uw0.data(), sizeof(float4) * uw0.size(), cudaMemcpyHostToDevice, stream_));
         CK(cudaStreamSynchronize(stream_));
     }
-    if ((any_twowall_ || any_wallc_) && (st = dalloc(&b_.wall_ext, (size_t)nrep * 8))) return st;
+    if (any_twowall_ || any_wallc_) {
+        if ((st = dalloc(&b_.wall_ext, (size_t)nrep * 8))) return st;
+        k_wall_reset<<<(nrep * 8 + 255) / 256, 256, 0, stream_>>>(step_args(b_, P_, nmax_, maxb_, nrep));
+        CK(cudaGetLastError());
+    }
     std::vector<RepState> rs(nrep);
     for (auto& s : rs) {
         memset(&s, 0, sizeof(s));
@@ -949,15 +955,18 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
         pdl_launch(k_fix_sums<1>, gp, 256, s, sa);
         pdl_launch(k_fix_reduce<1>, gr, 256, s, sa);
     }
-    if (any_wallc_) {
-        // wall_contact computes: wall extents of the end-of-step positions
-        pdl_launch(k_wall_reset<1>, gr, 256, s, sa);
-        pdl_launch(k_wall_extent<1>, gp, 256, s, sa);
-    }
-    if (small && !any_twowall_) {
-        // the step's bookkeeping runs in the integrate's last block
-        if (ext()) pdl_launch(k_integrate_adv<true>, gp, 256, s, sa);
-        else pdl_launch(k_integrate_adv<false>, gp, 256, s, sa);
+    // wall_contact computes: wall extents of the end-of-step positions
+    if (any_wallc_) pdl_launch(k_wall_extent, gp, 256, s, sa);
+    if (small) {
+        // the integrate in one launch, the step's bookkeeping in the last block of the step
+        if (any_twowall_) {
+            pdl_launch(k_integrate<true>, gp, 256, s, sa);
+            pdl_launch(k_two_wall<true>, gp, 256, s, sa);
+        } else if (ext()) {
+            pdl_launch(k_integrate_adv<true>, gp, 256, s, sa);
+        } else {
+            pdl_launch(k_integrate_adv<false>, gp, 256, s, sa);
+        }
         return;
     }
     if (ext()) {
@@ -967,17 +976,8 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
         pdl_launch(k_integrate_nolog<false>, gp, 256, s, sa);
         pdl_launch(k_integrate_logsteps<false>, std::min(gp, 148 * 4), 256, s, sa);
     }
-    if (any_twowall_) enqueue_two_wall(s, sa);
+    if (any_twowall_) pdl_launch(k_two_wall<false>, gp, 256, s, sa);
     pdl_launch(k_advance, (nrep * 32 + 255) / 256, 256, s, sa);
-}
-
-// fix two_wall after a drift: wall extents, then the reflection of the group
-void Engine::enqueue_two_wall(cudaStream_t s, const StepArgs& sa)
-{
-    const int gp = (P_ + 255) / 256, gr = ((int)reps_.size() + 255) / 256;
-    pdl_launch(k_wall_reset<0>, gr, 256, s, sa);
-    pdl_launch(k_wall_extent<0>, gp, 256, s, sa);
-    pdl_launch(k_two_wall, gp, 256, s, sa);
 }
 
 void Engine::enqueue_integrate_initial(cudaStream_t s)
@@ -986,7 +986,11 @@ void Engine::enqueue_integrate_initial(cudaStream_t s)
     sa.mode = 1;
     if (ext()) k_integrate<true><<<(P_ + 255) / 256, 256, 0, s>>>(sa);
     else k_integrate<false><<<(P_ + 255) / 256, 256, 0, s>>>(sa);
-    if (any_twowall_) enqueue_two_wall(s, sa);
+    if (any_twowall_) {
+        // the integrate has taken the wall extents; they are reset for the step's own
+        pdl_launch(k_two_wall<false>, (P_ + 255) / 256, 256, s, sa);
+        pdl_launch(k_wall_reset, (sa.nrep * 8 + 255) / 256, 256, s, sa);
+    }
 }
 
 // The tile table of pair schedule 11: the tiles of every replica (edge^3 home cells,

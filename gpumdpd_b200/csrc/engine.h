@@ -214,7 +214,6 @@ private:
     bool any_motion_ = false, any_twowall_ = false, any_wallc_ = false;  // fix move/wall_reflect, two_wall, wall_contact
     // the integrate variant with group fixes and computes
     bool ext() const { return any_spring_ || any_eos_ || any_gc_ || any_motion_ || any_twowall_; }
-    void enqueue_two_wall(cudaStream_t s, const ::StepArgs& sa);
     std::vector<int> gc_ring_base_;               // first compute ring of each replica
     bool zero_pending_ = true;
     bool force_build_ = false;  // the next run starts with a list build (after a restart)

@@ -922,6 +922,44 @@ __global__ void __launch_bounds__(DPD_FLAT_WARPS * 32, MINB) k_build_pair(StepAr
 }
 
 // ---------------------------------------------------------------------------------
+// Wall extents: the maximum position of a lo-wall group and the minimum of a hi-wall
+// group along the wall axis (src/fix/fix_two_wall.cu:145-180 and
+// src/compute/compute_wall_contact.cu:186-225 take them with thrust max/min_element), as one
+// atomic per warp on order-preserving ints.  Those of fix two_wall are taken by the integrate,
+// from the drifted positions it holds; the step's bookkeeping resets them for the next step.
+__device__ __forceinline__ void wall_extents(const StepArgs& a, const RepDesc& d, const int r, const bool real,
+                                             const float4& p, const int t0)
+{
+    const FixDesc& fd = a.fix[r];
+    for (int k = 0; k < fd.n_twowall; k++) {  // warp-uniform
+        const int q = fd.tw_dir[k];
+        const bool inlo = real && ((fd.tw_lo[k] >> t0) & 1u), inhi = real && ((fd.tw_hi[k] >> t0) & 1u);
+        const float xw = (inlo || inhi) ? wrapped_coord(d, fd.L[q], p, q) : 0.0f;
+        const int mx = __reduce_max_sync(0xffffffffu, inlo ? ford(xw) : INT_MIN);
+        const int mn = __reduce_min_sync(0xffffffffu, inhi ? ford(xw) : INT_MAX);
+        if ((threadIdx.x & 31) == 0) {
+            if (mx != INT_MIN) atomicMax(&a.wall_ext[r * 8 + 2 * k], mx);
+            if (mn != INT_MAX) atomicMin(&a.wall_ext[r * 8 + 2 * k + 1], mn);
+        }
+    }
+}
+
+// entry k of a replica's extents without any atom: two_wall pairs (max, min), then wall_contact
+__device__ __forceinline__ void wall_reset(const StepArgs& a, const int r, const int k)
+{
+    bool lo = (k & 1) == 0;
+    if (k >= 4) lo = !a.gc || a.gc[r * DPD_MAX_GC + k - 4].wall_side > 0;
+    a.wall_ext[r * 8 + k] = ford(lo ? -INFINITY : INFINITY);
+}
+
+__global__ void k_wall_reset(StepArgs a)
+{
+    griddep_wait();
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < 8 * a.nrep) wall_reset(a, q >> 3, q & 7);
+}
+
+// ---------------------------------------------------------------------------------
 // Velocity Verlet, src/fix/fix_nve.cu:30-152, fused: final half kick of step n (and
 // the thermo sums of step n), then initial half kick + drift of step n+1, the
 // displacement check for the next list build (src/force/neigh_list.cu:483-514), and
@@ -1136,6 +1174,7 @@ __device__ __forceinline__ void integrate_slot(const StepArgs& a, const int s, W
             }
             velp[s] = v;
         }
+        if (EXT && a.fix && active && init && a.fix[r].n_twowall) wall_extents(a, d, r, work, p, type0_of(v.w));
     }
     // `log` is warp-uniform (a warp holds one replica): a warp-level flush, no barrier
     if (a.mode == 0 && log) {
@@ -1190,32 +1229,8 @@ __global__ void __launch_bounds__(256) k_integrate_logsteps(StepArgs a)
 }
 
 // ---------------------------------------------------------------------------------
-// Wall extents: the maximum position of a lo-wall group and the minimum of a hi-wall
-// group along the wall axis (src/fix/fix_two_wall.cu:145-180 and
-// src/compute/compute_wall_contact.cu:186-225 take them with thrust max/min_element).
-// PH 0: the two_wall groups, after the drift; PH 1: the wall groups of wall_contact
-// computes due this step, before the integrate (the end-of-step positions).
-template <int PH>
-__global__ void k_wall_reset(StepArgs a)
-{
-    griddep_wait();
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= a.nrep) return;
-    int* e = a.wall_ext + r * 8;
-    if (PH == 0) {
-        for (int k = 0; k < 2; k++) {
-            e[2 * k] = ford(-INFINITY);
-            e[2 * k + 1] = ford(INFINITY);
-        }
-    } else {
-        for (int k = 0; k < DPD_MAX_GC; k++) {
-            const bool lo = !a.gc || a.gc[r * DPD_MAX_GC + k].wall_side > 0;
-            e[4 + k] = ford(lo ? -INFINITY : INFINITY);
-        }
-    }
-}
-
-template <int PH>
+// The wall groups of the wall_contact computes due this step, before the integrate (the
+// end-of-step positions).
 __global__ void __launch_bounds__(256) k_wall_extent(StepArgs a)
 {
     griddep_wait();
@@ -1225,6 +1240,9 @@ __global__ void __launch_bounds__(256) k_wall_extent(StepArgs a)
     const RepState st = a.rstate[r];
     if (!rep_active(st)) return;
     const RepDesc& d = a.reps[r];
+    if (!a.gc || a.mode != 0 || !d.gc_n) return;
+    const int due = gc_due(a, d, st, r);
+    if (!due) return;
     const int lane = threadIdx.x & 31;
     const int par = *a.parity;
     const bool real = s < d.p_end;
@@ -1234,35 +1252,17 @@ __global__ void __launch_bounds__(256) k_wall_extent(StepArgs a)
         p = a.buf.pos[par][s];
         t0 = type0_of(a.buf.vel[par][s].w);
     }
-    if (PH == 0) {
-        if (!a.fix) return;
-        const FixDesc& fd = a.fix[r];
-        for (int k = 0; k < fd.n_twowall; k++) {
-            const int q = fd.tw_dir[k];
-            const bool inlo = real && ((fd.tw_lo[k] >> t0) & 1u), inhi = real && ((fd.tw_hi[k] >> t0) & 1u);
-            const float xw = (inlo || inhi) ? wrapped_coord(d, fd.L[q], p, q) : 0.0f;
-            const int mx = __reduce_max_sync(0xffffffffu, inlo ? ford(xw) : INT_MIN);
-            const int mn = __reduce_min_sync(0xffffffffu, inhi ? ford(xw) : INT_MAX);
-            if (lane == 0) {
-                if (mx != INT_MIN) atomicMax(&a.wall_ext[r * 8 + 2 * k], mx);
-                if (mn != INT_MAX) atomicMin(&a.wall_ext[r * 8 + 2 * k + 1], mn);
-            }
-        }
-    } else {
-        if (!a.gc || a.mode != 0 || !d.gc_n) return;
-        const int due = gc_due(a, d, st, r);
-        for (int k = 0; k < d.gc_n; k++) {
-            const GCDesc& g = a.gc[r * DPD_MAX_GC + k];
-            if (g.kind != 5 || !((due >> k) & 1)) continue;
-            const bool in = real && ((g.wall_mask >> t0) & 1u);
-            const float xw = in ? wrapped_coord(d, g.L[g.wall_dir], p, g.wall_dir) : 0.0f;
-            if (g.wall_side > 0) {
-                const int mx = __reduce_max_sync(0xffffffffu, in ? ford(xw) : INT_MIN);
-                if (lane == 0 && mx != INT_MIN) atomicMax(&a.wall_ext[r * 8 + 4 + k], mx);
-            } else {
-                const int mn = __reduce_min_sync(0xffffffffu, in ? ford(xw) : INT_MAX);
-                if (lane == 0 && mn != INT_MAX) atomicMin(&a.wall_ext[r * 8 + 4 + k], mn);
-            }
+    for (int k = 0; k < d.gc_n; k++) {
+        const GCDesc& g = a.gc[r * DPD_MAX_GC + k];
+        if (g.kind != 5 || !((due >> k) & 1)) continue;
+        const bool in = real && ((g.wall_mask >> t0) & 1u);
+        const float xw = in ? wrapped_coord(d, g.L[g.wall_dir], p, g.wall_dir) : 0.0f;
+        if (g.wall_side > 0) {
+            const int mx = __reduce_max_sync(0xffffffffu, in ? ford(xw) : INT_MIN);
+            if (lane == 0 && mx != INT_MIN) atomicMax(&a.wall_ext[r * 8 + 4 + k], mx);
+        } else {
+            const int mn = __reduce_min_sync(0xffffffffu, in ? ford(xw) : INT_MAX);
+            if (lane == 0 && mn != INT_MAX) atomicMin(&a.wall_ext[r * 8 + 4 + k], mn);
         }
     }
 }
@@ -1270,10 +1270,8 @@ __global__ void __launch_bounds__(256) k_wall_extent(StepArgs a)
 // fix two_wall, post_integrate (src/fix/fix_two_wall.cu:84-125, 183-200): group atoms
 // below the lo wall's maximum or above the hi wall's minimum are mirrored back with the
 // normal velocity reversed; then the list-rebuild check of the moved atoms.
-__global__ void __launch_bounds__(256) k_two_wall(StepArgs a)
+__device__ __forceinline__ void two_wall_slot(const StepArgs& a, const int s)
 {
-    griddep_wait();
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.P || !a.fix) return;
     const int r = a.warp_rep[s >> 5];
     const RepState st = a.rstate[r];
@@ -1643,19 +1641,17 @@ __global__ void k_advance(StepArgs a)
     griddep_wait();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = g >> 5;
-    if (r < a.nrep) advance_rep(a, r, threadIdx.x & 31);
+    if (r < a.nrep) {
+        advance_rep(a, r, threadIdx.x & 31);
+        if (a.wall_ext && (threadIdx.x & 31) < 8) wall_reset(a, r, threadIdx.x & 31);
+    }
     if (g == 0) advance_phase(a);
 }
 
-// Small grids, where a launch costs more than the work: the whole velocity-Verlet step
-// (any step, logged or not) in one launch whose last block (a ticket counter) also does
-// the step's bookkeeping of every replica.  Every block's writes and FP64 sums are done
-// and fenced before it takes its ticket.
-template <bool EXT>
-__global__ void __launch_bounds__(256) k_integrate_adv(StepArgs a)
+// The step's bookkeeping of every replica by the last block of a launch (a ticket counter).
+// Every block's writes and FP64 sums are done and fenced before it takes its ticket.
+__device__ __forceinline__ void advance_by_last_block(const StepArgs& a)
 {
-    griddep_wait();
-    integrate_slot<2, EXT>(a, blockIdx.x * blockDim.x + threadIdx.x);
     __shared__ bool last;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1665,12 +1661,35 @@ __global__ void __launch_bounds__(256) k_integrate_adv(StepArgs a)
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int r = threadIdx.x >> 5; r < a.nrep; r += blockDim.x >> 5) advance_rep(a, r, threadIdx.x & 31);
+    for (int r = threadIdx.x >> 5; r < a.nrep; r += blockDim.x >> 5) {
+        advance_rep(a, r, threadIdx.x & 31);
+        if (a.wall_ext && (threadIdx.x & 31) < 8) wall_reset(a, r, threadIdx.x & 31);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         advance_phase(a);
         *a.ticket = 0u;
     }
+}
+
+// fix two_wall after the drift; ADV (small grids): with the step's bookkeeping
+template <bool ADV>
+__global__ void __launch_bounds__(256) k_two_wall(StepArgs a)
+{
+    griddep_wait();
+    two_wall_slot(a, blockIdx.x * blockDim.x + threadIdx.x);
+    if (ADV) advance_by_last_block(a);
+}
+
+// Small grids, where a launch costs more than the work: the whole velocity-Verlet step
+// (any step, logged or not) in one launch whose last block also does the step's bookkeeping
+// of every replica.
+template <bool EXT>
+__global__ void __launch_bounds__(256) k_integrate_adv(StepArgs a)
+{
+    griddep_wait();
+    integrate_slot<2, EXT>(a, blockIdx.x * blockDim.x + threadIdx.x);
+    advance_by_last_block(a);
 }
 
 // ---------------------------------------------------------------------------------
