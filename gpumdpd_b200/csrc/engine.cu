@@ -55,7 +55,8 @@ Engine::~Engine()
     if (stream_) cudaStreamSynchronize(stream_);
     for (void* p : allocs_) cudaFreeAsync(p, stream_);
     if (stream_) cudaStreamSynchronize(stream_);
-    if (h_block_) cudaFreeHost(h_block_);
+    for (void* p : {(void*)h_pos_, (void*)h_vel_, (void*)h_frc_, (void*)h_img_, (void*)h_rs_, (void*)h_rows_})
+        if (p) cudaFreeHost(p);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -567,17 +568,15 @@ int Engine::alloc_and_upload()
 
 int Engine::staging()
 {
-    if (h_block_) return DPD_OK;
-    const size_t arr = sizeof(float4) * (size_t)P_;
-    const size_t rs = (sizeof(RepState) * reps_.size() + 127) / 128 * 128;
-    // 512: the rows of a state read-back start on 128-byte lines
-    CK(cudaMallocHost((void**)&h_block_, 4 * arr + 512 + rs + sizeof(double) * (DPD_ROWS_PINNED * DPD_THERMO_FIELDS + 1)));
-    h_pos_ = (float4*)h_block_;
-    h_vel_ = h_pos_ + P_;
-    h_frc_ = h_vel_ + P_;
-    h_img_ = (int4*)(h_frc_ + P_);
-    h_rs_ = (RepState*)(h_block_ + 4 * arr + 512);
-    h_rows_ = (double*)((char*)h_rs_ + rs);
+    if (h_pos_) return DPD_OK;
+    // separate blocks: the driver serves pinned memory below a megabyte from what it holds, and
+    // takes milliseconds for larger blocks
+    CK(cudaMallocHost((void**)&h_vel_, sizeof(float4) * P_));
+    CK(cudaMallocHost((void**)&h_frc_, sizeof(float4) * P_));
+    CK(cudaMallocHost((void**)&h_img_, sizeof(int4) * P_));
+    CK(cudaMallocHost((void**)&h_rs_, sizeof(RepState) * reps_.size()));
+    CK(cudaMallocHost((void**)&h_rows_, sizeof(double) * (DPD_ROWS_PINNED * DPD_THERMO_FIELDS + 1)));
+    CK(cudaMallocHost((void**)&h_pos_, 3 * sizeof(double) * (size_t)P_));  // float4 per slot, or FP64 rows
     return DPD_OK;
 }
 
@@ -1085,9 +1084,11 @@ int Engine::refresh_list()
     return DPD_OK;
 }
 
-// steps of a graph launch: 24000 particles take 32.1 us a step with 1, 29.2 with 8 (3000: 23.7 and
-// 20.8; 192000: 71.9 and 70.4); making both graphs takes 0.39 ms against 0.14
+// Steps of a graph launch: 24000 particles take 32.1 us a step with 1, 29.2 with 8 (3000: 23.7
+// and 20.8; 192000: 71.9 and 70.4).  Making the graph of 8 takes 0.26 ms, what it saves in about
+// 120 steps, so an engine makes it for the run that takes it past DPD_GRAPH_AFTER steps.
 #define DPD_GRAPH_STEPS 8
+#define DPD_GRAPH_AFTER 120
 
 int Engine::capture_steps(int n, cudaGraphExec_t* out)
 {
@@ -1111,7 +1112,10 @@ int Engine::build_graph()
 {
     int e = prepare_tiles();
     if (!e) e = capture_steps(1, &graph_);
-    if (!e) e = capture_steps(DPD_GRAPH_STEPS, &graph_many_);
+    if (graph_many_) {
+        cudaGraphExecDestroy(graph_many_);
+        graph_many_ = nullptr;
+    }
     return e;
 }
 
@@ -1155,7 +1159,11 @@ int Engine::run_async(uint32_t nsteps)
         if (!zero) enqueue_integrate_initial(stream_);
         CK(cudaGetLastError());
         uint32_t left = end - s + 1;
-        for (; left >= DPD_GRAPH_STEPS; left -= DPD_GRAPH_STEPS) CK(cudaGraphLaunch(graph_many_, stream_));
+        if (!graph_many_ && left >= DPD_GRAPH_STEPS && (uint64_t)s + left > DPD_GRAPH_AFTER) {
+            const int e = capture_steps(DPD_GRAPH_STEPS, &graph_many_);
+            if (e) return e;
+        }
+        for (; graph_many_ && left >= DPD_GRAPH_STEPS; left -= DPD_GRAPH_STEPS) CK(cudaGraphLaunch(graph_many_, stream_));
         for (; left > 0; left--) CK(cudaGraphLaunch(graph_, stream_));
         zero = false;
         // the host's step counter follows each segment, so a failed frame write leaves
@@ -1504,19 +1512,13 @@ int Engine::get_state(int rep, double* x, double* v, int* image, double* f)
     const int64_t n = d.n_real;
     int st = staging();
     if (st) return st;
-    // rows by tag in the pinned block, each array from a 128-byte line: 60 of its 64 bytes
-    // per slot
-    auto line = [](size_t b) { return (b + 127) / 128 * 128; };
+    // rows by tag in the pinned arrays
     StateOut o;
     for (int q = 0; q < 3; q++) o.L[q] = R.box_len[q];
-    size_t at = 0;
-    o.x = x ? (double*)(h_block_ + at) : nullptr;
-    if (x) at += line(sizeof(double) * 3 * n);
-    o.v = v ? (float*)(h_block_ + at) : nullptr;
-    if (v) at += line(sizeof(float) * 3 * n);
-    o.f = f ? (float*)(h_block_ + at) : nullptr;
-    if (f) at += line(sizeof(float) * 3 * n);
-    o.image = image ? (int*)(h_block_ + at) : nullptr;
+    o.x = x ? (double*)h_pos_ : nullptr;
+    o.v = v ? (float*)h_vel_ : nullptr;
+    o.f = f ? (float*)h_frc_ : nullptr;
+    o.image = image ? (int*)h_img_ : nullptr;
     o.bad = (int*)h_rows_;
     *o.bad = 0;
     k_state_out<<<(int)((n + 255) / 256), 256, 0, stream_>>>(step_args(b_, P_, nmax_, maxb_, (int)reps_.size()), rep, o);

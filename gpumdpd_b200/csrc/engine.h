@@ -220,9 +220,8 @@ private:
     bool ranks_dirty_ = false;  // new cell ranks (a changed cell order) wait for the next run
     uint32_t next_step_ = 0;
     std::vector<void*> allocs_;
-    char* h_block_ = nullptr;  // pinned staging, one block: the four arrays below (64 B per
-                               // slot, also the rows of a state read-back), the replica
-                               // states, and rows of a thermo read-back
+    // pinned staging: a float4 per slot each (h_pos_: or three doubles), also the rows by tag of
+    // a state read-back; the replica states; rows of a thermo read-back
     float4 *h_pos_ = nullptr, *h_vel_ = nullptr, *h_frc_ = nullptr;
     int4* h_img_ = nullptr;
     RepState* h_rs_ = nullptr;
