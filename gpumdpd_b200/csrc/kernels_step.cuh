@@ -759,14 +759,17 @@ __device__ __forceinline__ void pair_flat_warp(const StepArgs& a, const int s, W
             kb = 0;
             int* col = s_q[warp] + lane;
             // a round ends when a column might not take 4 more entries
-            while (__any_sync(0xffffffffu, k < kend) && !__any_sync(0xffffffffu, c > DPD_FLAT_COL - 4)) {
-                int ee[4];
-                float4 pp[4];
+            int ee[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) ee[u] = k + u < kend ? wl[(size_t)(k + u) * 32 + lane] : 0;
+            for (int u = 0; u < 4; u++) ee[u] = k + u < kend ? wl[(size_t)(k + u) * 32 + lane] : 0;
+            while (__any_sync(0xffffffffu, k < kend) && !__any_sync(0xffffffffu, c > DPD_FLAT_COL - 4)) {
+                int en[4];
+                float4 pp[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++)
                     if (k + u < kend) pp[u] = __ldg(pos + (ee[u] & DPD_J_MASK));
+#pragma unroll
+                for (int u = 0; u < 4; u++) en[u] = k + 4 + u < kend ? wl[(size_t)(k + 4 + u) * 32 + lane] : 0;
 #pragma unroll
                 for (int u = 0; u < 4; u++)
                     if (k + u < kend) {
@@ -778,6 +781,8 @@ __device__ __forceinline__ void pair_flat_warp(const StepArgs& a, const int s, W
                             c++;
                         }
                     }
+#pragma unroll
+                for (int u = 0; u < 4; u++) ee[u] = en[u];
                 k += 4;
             }
         }
