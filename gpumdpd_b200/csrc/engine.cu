@@ -979,15 +979,18 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     pdl_launch(k_advance, (nrep * 32 + 255) / 256, 256, s, sa);
 }
 
-void Engine::enqueue_integrate_initial(cudaStream_t s)
+// a continued run up to step `target`: the drift after the last step, with a pending list build
+void Engine::enqueue_begin(cudaStream_t s, uint32_t target)
 {
     StepArgs sa = step_args(b_, P_, nmax_, maxb_, (int)reps_.size());
     sa.mode = 1;
-    if (ext()) k_integrate<true><<<(P_ + 255) / 256, 256, 0, s>>>(sa);
-    else k_integrate<false><<<(P_ + 255) / 256, 256, 0, s>>>(sa);
+    const int gp = (P_ + 255) / 256, build = force_build_ ? 1 : 0;
+    if (ext()) k_integrate_begin<true><<<gp, 256, 0, s>>>(sa, b_.limit, target, build);
+    else k_integrate_begin<false><<<gp, 256, 0, s>>>(sa, b_.limit, target, build);
+    force_build_ = false;
     if (any_twowall_) {
         // the integrate has taken the wall extents; they are reset for the step's own
-        pdl_launch(k_two_wall<false>, (P_ + 255) / 256, 256, s, sa);
+        pdl_launch(k_two_wall<false>, gp, 256, s, sa);
         pdl_launch(k_wall_reset, (sa.nrep * 8 + 255) / 256, 256, s, sa);
     }
 }
@@ -1119,17 +1122,17 @@ int Engine::build_graph()
     return e;
 }
 
-// set the run target of every replica (absolute step), optionally mark the next
-// evaluation as a zero step and raise the list-build flag of the current phase
-__global__ void k_set_target(RepState* st, const uint32_t* limit, int nrep, uint32_t target, int zero,
-                             int set_build, int* build_flag, const uint32_t* phase)
+// the run target of every replica (absolute step) for a run that begins with a zero step and its
+// list build
+__global__ void k_begin_zero(RepState* st, const uint32_t* limit, int nrep, uint32_t target, int* build_flag,
+                             const uint32_t* phase)
 {
     int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < nrep) {
         st[r].target = min(target, limit[r]);
-        if (zero) st[r].zero_pending = 1;
+        st[r].zero_pending = 1;
     }
-    if (r == 0 && set_build) build_flag[(*phase) & 1] = 1;
+    if (r == 0) build_flag[(*phase) & 1] = 1;
 }
 
 int Engine::run_async(uint32_t nsteps)
@@ -1153,10 +1156,12 @@ int Engine::run_async(uint32_t nsteps)
             if (e) return e;
             ranks_dirty_ = false;
         }
-        k_set_target<<<g, 256, 0, stream_>>>(b_.rstate, b_.limit, nrep, end, zero ? 1 : 0,
-                                             zero || force_build_ ? 1 : 0, b_.build_flag, b_.phase);
-        force_build_ = false;
-        if (!zero) enqueue_integrate_initial(stream_);
+        if (zero) {
+            k_begin_zero<<<g, 256, 0, stream_>>>(b_.rstate, b_.limit, nrep, end, b_.build_flag, b_.phase);
+            force_build_ = false;
+        } else {
+            enqueue_begin(stream_, end);
+        }
         CK(cudaGetLastError());
         uint32_t left = end - s + 1;
         if (!graph_many_ && left >= DPD_GRAPH_STEPS && (uint64_t)s + left > DPD_GRAPH_AFTER) {
@@ -1256,7 +1261,6 @@ int Engine::time_steps(uint32_t nsteps, double* total_ms, double* pair_ms, int64
         if (e) return e;
     }
     if (nsteps == 0) return DPD_E_ARG;
-    const int nrep = (int)reps_.size();
     std::vector<cudaEvent_t> ev(2 * (size_t)nsteps + 2);
     for (auto& e : ev) CK(cudaEventCreate(&e));
     const uint32_t target = next_step_ - 1 + nsteps;
@@ -1265,11 +1269,7 @@ int Engine::time_steps(uint32_t nsteps, double* total_ms, double* pair_ms, int64
         if (e) return e;
         ranks_dirty_ = false;
     }
-    // a pending list build (new cell ranks, a restart) comes first, as in a run
-    k_set_target<<<(nrep + 255) / 256, 256, 0, stream_>>>(b_.rstate, b_.limit, nrep, target, 0, force_build_ ? 1 : 0,
-                                                          b_.build_flag, b_.phase);
-    force_build_ = false;
-    enqueue_integrate_initial(stream_);
+    enqueue_begin(stream_, target);
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     for (uint32_t k = 0; k < nsteps; k++) enqueue_step(stream_, ev[2 * k + 2], ev[2 * k + 3]);

@@ -974,8 +974,11 @@ __global__ void k_wall_reset(StepArgs a)
 // registers); 1 = logged mode-0 steps only.  0 and 1 together cover every slot once.
 // A step is logged when the thermo or (EXT) a group compute is due.  EXT adds the group
 // fixes and the group computes.
+// limit (the first drift of a run): the replica's last step is min(target, limit[r]), which this
+// launch also writes, so a run starts without a launch that does only that.
 template <int LOGM, bool EXT>
-__device__ __forceinline__ void integrate_slot(const StepArgs& a, const int s, WarpAcc<10>* keep = nullptr)
+__device__ __forceinline__ void integrate_slot(const StepArgs& a, const int s, WarpAcc<10>* keep = nullptr,
+                                               const uint32_t* limit = nullptr, const uint32_t target = 0)
 {
     int r = -1;
     bool log = false;
@@ -996,8 +999,12 @@ __device__ __forceinline__ void integrate_slot(const StepArgs& a, const int s, W
         const float4 f = a.force4[s];
         float4 p = posp[s];
         r = a.warp_rep[s >> 5];
-        const RepState st = a.rstate[r];
+        RepState st = a.rstate[r];
         const RepDesc& d = a.reps[r];
+        if (limit) {
+            st.target = min(target, limit[r]);
+            if (s == d.p_begin) a.rstate[r].target = st.target;
+        }
         const bool active = rep_active(st);
         const bool work = active && s < d.p_end;
         const bool fin = a.mode == 0 && !st.zero_pending;
@@ -1201,6 +1208,16 @@ __global__ void __launch_bounds__(256) k_integrate(StepArgs a)
 {
     griddep_wait();
     integrate_slot<2, EXT>(a, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// The drift that a continued run begins with (a.mode 1): the replicas' last steps, and the list
+// build flag of the current phase when a build is due whatever the displacements
+template <bool EXT>
+__global__ void __launch_bounds__(256) k_integrate_begin(StepArgs a, const uint32_t* limit, uint32_t target,
+                                                         int set_build)
+{
+    if (set_build && blockIdx.x == 0 && threadIdx.x == 0) a.build_flag[*a.phase & 1] = 1;
+    integrate_slot<2, EXT>(a, blockIdx.x * blockDim.x + threadIdx.x, nullptr, limit, target);
 }
 
 template <bool EXT>
