@@ -912,7 +912,7 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     StepArgs sm = sa;  // mDPD: the force pass takes the density pass's list
     sm.nlist = b_.near_list;
     sm.ncount = b_.near_count;
-    if (any_mdpd_) pdl_launch(k_density, gp, 256, s, sa, b_.near_list, b_.near_count);
+    if (any_mdpd_) pdl_launch(k_density, (P_ + 32 * DPD_DENS_WARPS - 1) / (32 * DPD_DENS_WARPS), 32 * DPD_DENS_WARPS, s, sa, b_.near_list, b_.near_count);
     if (ev0) cudaEventRecordWithFlags(ev0, s, cudaEventRecordExternal);
     if (tile) {
         const TileArgs ta{b_.tile_rep, b_.tile_code, ntiles_, tile_edge_, tile_smax_, tile_hc_};
@@ -1967,7 +1967,7 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
     StepArgs sm = sa;
     sm.nlist = b_.near_list;
     sm.ncount = b_.near_count;
-    if (any_mdpd_) pdl_launch(k_density, gp, 256, stream_, sa, b_.near_list, b_.near_count);
+    if (any_mdpd_) pdl_launch(k_density, (P_ + 32 * DPD_DENS_WARPS - 1) / (32 * DPD_DENS_WARPS), 32 * DPD_DENS_WARPS, stream_, sa, b_.near_list, b_.near_count);
     const bool peratom = d_pe || d_virial;
     // this entry builds the list itself: schedule 11 (no list) runs as the default 8
     int pv = tune_.pair_variant == 11 ? 8 : tune_.pair_variant;

@@ -135,74 +135,90 @@ __device__ __forceinline__ void pair_disp(const float4* tab, int ent, float4 pi,
 // The pass looks at every entry's distance anyway, so it also writes the entries inside the
 // largest cutoff to a list of their own (near_list, near_count), which the force pass takes
 // without gathering and testing the others again (384k slab, rho 6, skin 0.3: 27 entries a
-// particle, 12.6 inside).  Latency of the gathers bounds it.  On that slab a step went from 332
-// to 292 us: this pass 96 -> 90 with the list written beside (one gather in flight and the
-// neighbour's type read for every entry before), the force pass 114 -> 75.
-__global__ void __launch_bounds__(256) k_density(StepArgs a, int* near_list, int* near_count)
+// particle, 12.6 inside).  The entries inside rd (5 of 27) wait in the lane's column of a shared
+// queue and are evaluated together: beside the test some lane of the warp has a hit at nearly
+// every entry.  Issue and the gathers' latency bound it (51% of the issue slots before the
+// queue, 13 of 32 lanes).  Step of that slab: 332 us with one gather in flight, every type read
+// and no near list; 292 with them (this pass 96 -> 90, the force pass 114 -> 75); 278 with the
+// queue of 16 columns (12: 283, 8: 286).
+#define DPD_DENS_WARPS 4  // warps per block
+#define DPD_DENS_COL 16   // queued entries per particle and round
+__global__ void __launch_bounds__(DPD_DENS_WARPS * 32) k_density(StepArgs a, int* near_list, int* near_count)
 {
     griddep_wait();
-    __shared__ float4 tab[8][27];
+    __shared__ float4 tab[DPD_DENS_WARPS][27];
+    __shared__ int2 s_q[DPD_DENS_WARPS][DPD_DENS_COL * 32];  // entries inside rd: slot and r^2
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.P) return;
+    if (s >= a.P) return;  // warp-uniform
     const int r = a.warp_rep[s >> 5];
     const RepDesc& d = a.reps[r];
     if (!rep_active(a.rstate[r]) || d.style != 1) return;  // warp-uniform
     fill_shift(tab[warp], d, lane);
     __syncwarp();
-    if (s >= d.p_end) {
-        near_count[s] = 0;
-        return;
-    }
+    if (s >= d.p_end) near_count[s] = 0;
     const int par = *a.parity;
     const float4* pos = a.buf.pos[par];
     const float4* vel = a.buf.vel[par];
     const float4 pi = pos[s];
     const int ti = type0_of(vel[s].w);
     const float4* crow = a.coeff + d.coeff_off + ti * d.ntypes * 3;
-    const int n = min(a.ncount[s], a.nmax);
+    const int n = s < d.p_end ? min(a.ncount[s], a.nmax) : 0;
     const size_t first = ((size_t)(s >> 5) * a.nmax) * 32 + lane;
     const int* lst = a.nlist + first;
     int* near = near_list + first;
     const float rcmax2 = d.rcmax2, rdmax2 = d.rdmax2;
     float rho_i = 0.0f;
-    int c = 0;
-    for (int k = 0; k < n; k += 4) {
-        int ee[4];
-        float4 pj[4];
+    int c = 0, k = 0;
+    int2* col = s_q[warp] + lane;
+    while (__any_sync(0xffffffffu, k < n)) {
+        // a round: entries until a column might not take 4 more
+        int m = 0;
+        while (__any_sync(0xffffffffu, k < n) && !__any_sync(0xffffffffu, m > DPD_DENS_COL - 4)) {
+            int ee[4];
+            float4 pj[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) ee[u] = k + u < n ? __ldg(lst + (size_t)(k + u) * 32) : 0;
+            for (int u = 0; u < 4; u++) ee[u] = k + u < n ? __ldg(lst + (size_t)(k + u) * 32) : 0;
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (k + u < n) pj[u] = __ldg(pos + (ee[u] & DPD_J_MASK));
+            for (int u = 0; u < 4; u++)
+                if (k + u < n) pj[u] = __ldg(pos + (ee[u] & DPD_J_MASK));
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            if (k + u < n) {
-                float dx, dy, dz;
-                pair_disp(tab[warp], ee[u], pi, pj[u], dx, dy, dz);
-                const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-                if (r2 <= rcmax2) {
-                    near[(size_t)c * 32] = ee[u];
-                    c++;
-                }
-                if (r2 < rdmax2) {
-                    const int j = ee[u] & DPD_J_MASK;
-                    const int tj = type0_of(__ldg(&vel[j].w));
-                    const float4 c2 = __ldg(crow + tj * 3 + 2);
-                    if (r2 < c2.x) {
-                        const float4 c1 = __ldg(crow + tj * 3 + 1);
-                        const float rr = r2 * rsqrtf(fmaxf(r2, 1e-30f));
-                        const float wd = fmaxf(1.0f - rr * c1.w, 0.0f);
-                        const float add = c2.z * wd * wd;
-                        rho_i += add;
-                        atomicAdd(&a.rho[j], add);
+            for (int u = 0; u < 4; u++) {
+                if (k + u < n) {
+                    float dx, dy, dz;
+                    pair_disp(tab[warp], ee[u], pi, pj[u], dx, dy, dz);
+                    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+                    if (r2 <= rcmax2) {
+                        near[(size_t)c * 32] = ee[u];
+                        c++;
+                    }
+                    if (r2 < rdmax2) {
+                        col[m * 32] = make_int2(ee[u] & DPD_J_MASK, __float_as_int(r2));
+                        m++;
                     }
                 }
             }
+            k += 4;
+        }
+        for (int q = 0; q < m; q++) {
+            const int2 e = col[q * 32];
+            const float r2 = __int_as_float(e.y);
+            const int tj = type0_of(__ldg(&vel[e.x].w));
+            const float4 c2 = __ldg(crow + tj * 3 + 2);
+            if (r2 < c2.x) {
+                const float4 c1 = __ldg(crow + tj * 3 + 1);
+                const float rr = r2 * rsqrtf(fmaxf(r2, 1e-30f));
+                const float wd = fmaxf(1.0f - rr * c1.w, 0.0f);
+                const float add = c2.z * wd * wd;
+                rho_i += add;
+                atomicAdd(&a.rho[e.x], add);
+            }
         }
     }
-    near_count[s] = c;
-    atomicAdd(&a.rho[s], rho_i);
+    if (s < d.p_end) {
+        near_count[s] = c;
+        atomicAdd(&a.rho[s], rho_i);
+    }
 }
 
 // Bond forces computed by both partners (each takes its own side; energy and virial
