@@ -393,8 +393,9 @@ __device__ __forceinline__ void permute_slot(const BuildArgs& a, const int s)
 // The permutation.  FLIP (small grids, where a launch costs more than the work): the
 // last block to finish (a ticket counter) also flips the parity, counts the build of
 // every replica and resets the ticket.  Every block has read the parity before it takes
-// its ticket, and the list build that follows waits for the whole grid.  Large grids
-// leave the flip to k_flip: the ticket's fence in every block costs more than a launch.
+// its ticket (nothing else of it is read by the last block, so no fence), and the list build
+// that follows waits for the whole grid.  Large grids leave the flip to k_flip: their tickets
+// take as long as that launch.
 template <bool FLIP>
 __global__ void k_permute(BuildArgs a, int nrep)
 {
@@ -406,10 +407,7 @@ __global__ void k_permute(BuildArgs a, int nrep)
     if (s < a.P) a.ncount[s] = 0;  // k_build_wide counts with atomics
     __shared__ bool last;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(a.ticket, 1u) == gridDim.x - 1u;
-    }
+    if (threadIdx.x == 0) last = atomicAdd(a.ticket, 1u) == gridDim.x - 1u;
     __syncthreads();
     if (last) {
         for (int r = threadIdx.x; r < nrep; r += blockDim.x) a.rstate[r].nbuild++;

@@ -1687,18 +1687,19 @@ __global__ void k_advance(StepArgs a)
 }
 
 // The step's bookkeeping of every replica by the last block of a launch (a ticket counter).
-// Every block's writes and FP64 sums are done and fenced before it takes its ticket.
-__device__ __forceinline__ void advance_by_last_block(const StepArgs& a)
+// sums: the step has FP64 sums that the last block reads, so every block's are fenced before it
+// takes its ticket.  Otherwise the ticket only says that the block has read the step's state.
+__device__ __forceinline__ void advance_by_last_block(const StepArgs& a, const bool sums)
 {
     __shared__ bool last;
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
+        if (sums) __threadfence();
         last = atomicAdd(a.ticket, 1u) == gridDim.x - 1u;
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
+    if (sums) __threadfence();
     for (int r = threadIdx.x >> 5; r < a.nrep; r += blockDim.x >> 5) {
         advance_rep(a, r, threadIdx.x & 31);
         if (a.wall_ext && (threadIdx.x & 31) < 8) wall_reset(a, r, threadIdx.x & 31);
@@ -1716,7 +1717,7 @@ __global__ void __launch_bounds__(256) k_two_wall(StepArgs a)
 {
     griddep_wait();
     two_wall_slot(a, blockIdx.x * blockDim.x + threadIdx.x);
-    if (ADV) advance_by_last_block(a);
+    if (ADV) advance_by_last_block(a, true);
 }
 
 // Small grids, where a launch costs more than the work: the whole velocity-Verlet step
@@ -1727,7 +1728,7 @@ __global__ void __launch_bounds__(256) k_integrate_adv(StepArgs a)
 {
     griddep_wait();
     integrate_slot<2, EXT>(a, blockIdx.x * blockDim.x + threadIdx.x);
-    advance_by_last_block(a);
+    advance_by_last_block(a, EXT || a.nrep > 1 || (a.rstate[0].step % (uint32_t)a.reps[0].log_f) == 0u);
 }
 
 // ---------------------------------------------------------------------------------
