@@ -844,9 +844,15 @@ static void launch_pair(int variant, bool bonds, bool filt, int grid, cudaStream
     else launch_pair2<STYLE, false>(variant, filt, grid, s, a);
 }
 
+// Blocks of 256 slots up to which a thread per (slot, column group) builds the list: a step of
+// 24000 particles takes 25.2 us with it and 27.8 with a thread per (slot, stencil cell), of 81000
+// 43.4 and 44.6 with a thread per slot, of 192000 (750 blocks) 68.3 and 67.1.
+#define DPD_SPREAD_BLOCKS (148 * 3)
+
 // The list-build chain; every kernel returns at once unless this phase's flag is set.
-// linear: the device's cell ranks are those of cell order 0 when it runs.
-void Engine::enqueue_build(cudaStream_t s, bool list, bool wide, bool linear)
+// linear: the device's cell ranks are those of cell order 0 when it runs; spread: several
+// threads per slot build the list under that order (needs k_permute<true>).
+void Engine::enqueue_build(cudaStream_t s, bool list, bool wide, bool linear, bool spread)
 {
     const int nrep = (int)reps_.size();
     BuildArgs ba = build_args(b_, P_, C_, nmax_, maxb_);
@@ -876,6 +882,8 @@ void Engine::enqueue_build(cudaStream_t s, bool list, bool wide, bool linear)
             const StepArgs sa = step_args(b_, P_, nmax_, maxb_, nrep);
             const TileArgs ta{b_.tile_rep, b_.tile_code, ntiles_, tile_edge_, tile_smax_, 0};
             pdl_launch_smem(k_tile_build<5>, ntiles_, 256, tile_smem_bytes(tile_smax_, 0), s, sa, ta, ba);
+        } else if (tune_.build_variant == 5 && linear && spread) {
+            pdl_launch(k_build_lin5, (5 * P_ + 127) / 128, 128, s, ba);
         } else if (wide && gp <= 148 * 8) pdl_launch(k_build_wide, (14 * P_ + 255) / 256, 256, s, ba);
         else if (tune_.build_variant == 1) pdl_launch(k_build_nlist_s<6>, gp, 256, s, ba);
         else if (tune_.build_variant == 2) pdl_launch(k_build_nlist_s<8>, gp, 256, s, ba);
@@ -908,7 +916,8 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     const bool fused = variant == 6 && !any_mdpd_;
     enqueue_build(s, !fused && !tile,
                   (tiny && (tune_.build_variant == 0 || tune_.build_variant == 5)) || tune_.build_variant == 3,
-                  tune_.cell_order == 0);  // a run uploads the ranks of the tuning first
+                  tune_.cell_order == 0,  // a run uploads the ranks of the tuning first
+                  small && tune_.launch_mode != 3 && gp <= DPD_SPREAD_BLOCKS);
     StepArgs sm = sa;  // mDPD: the force pass takes the density pass's list
     sm.nlist = b_.near_list;
     sm.ncount = b_.near_count;
@@ -1963,7 +1972,7 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
     const bool tiny = small && gp <= 148 && tune_.launch_mode != 3;
     // a changed cell order waits for the next run: until then the device keeps the old ranks
     enqueue_build(stream_, true, (tiny && (tune_.build_variant == 0 || tune_.build_variant == 5)) || tune_.build_variant == 3,
-                  tune_.cell_order == 0 && !ranks_dirty_);
+                  tune_.cell_order == 0 && !ranks_dirty_, small && tune_.launch_mode != 3 && gp <= DPD_SPREAD_BLOCKS);
     StepArgs sm = sa;
     sm.nlist = b_.near_list;
     sm.ncount = b_.near_count;

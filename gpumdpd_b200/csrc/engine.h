@@ -178,7 +178,7 @@ private:
     int alloc_and_upload();
     int upload_particles();
     void enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1);
-    void enqueue_build(cudaStream_t s, bool list, bool wide, bool linear);
+    void enqueue_build(cudaStream_t s, bool list, bool wide, bool linear, bool spread);
     void enqueue_begin(cudaStream_t s, uint32_t target);
     int build_graph();
     // pair schedule 11 (the cell-tile kernel, DPD engines): the tile table and staging

@@ -15,15 +15,17 @@ def _check(oracle_mod, e, n):
     assert set(map(tuple, got.tolist())) == set(map(tuple, ref.tolist()))
 
 
+# launch mode 1: a thread per slot; 0: one per slot and column group.
 # boxes of 3 cells (a column is 3 cells, both ends wrap), ranges of more than 32 and of exactly
 # few slots, empty cells, a last cell that ends with the slots
+@pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("L,rho,skin", [(3.0, 3.0, 0.0), (3.1, 14.0, 0.0), (5.3, 9.0, 0.3), (8.2, 0.5, 0.0),
                                         (9.9, 3.0, 0.3), (6.0, 40.0, 0.0)])
-def test_linear_build_gives_the_oracle_pairs(oracle_mod, L, rho, skin):
+def test_linear_build_gives_the_oracle_pairs(oracle_mod, L, rho, skin, mode):
     from gpumdpd_b200 import Engine, inputs
     s = inputs.plain_dpd(L=L, rho=rho, seed=61, dt=0.005, nsteps=5, skin=skin, max_rho=80.0)
     e = Engine(s.run_in, system=s.c_system())
-    e.set_tuning(launch_mode=1)
+    e.set_tuning(launch_mode=mode)
     e.run(0)
     _check(oracle_mod, e, s.n)
     if skin == 0.0:  # a list every step, of that step's positions
