@@ -1658,9 +1658,12 @@ __device__ __forceinline__ void advance_rep(const StepArgs& a, const int r, cons
                     a.gc_count[g.ring]++;
                 }
             }
-            st.step++;
-            st.zero_pending = 0;
-            a.rstate[r] = st;
+            // only what changes here: the status word belongs to the kernels that raise it, and
+            // another block of this launch may have done so after this thread read the state
+            RepState& out = a.rstate[r];
+            out.step = st.step + 1u;
+            out.zero_pending = 0;
+            out.nlog = st.nlog;
         }
     }
 }
