@@ -87,9 +87,8 @@ typedef struct dpd_tuning {
     int pair_variant;      /* 0 = thread per particle, 1-3 = warp pair-queue,
                               4-5 = flattened warp schedule (small skins),
                               6 = flattened with the list build fused (DPD),
-                              7-8 = flattened, log and non-log steps split (8 is
-                              the default), 9 = as 8 with the i-side forces summed
-                              per owner in the warp before the reduction,
+                              7-9 = flattened, log and non-log steps split (8 is
+                              the default; 7 and 9 run the same kernels),
                               10 = one thread per list entry, 11 = no neighbour
                               list: a CTA per tile of cells stages the tile's
                               neighbourhood in shared memory and evaluates its
@@ -104,10 +103,11 @@ typedef struct dpd_tuning {
                               8 blocks/SM; 3 = a thread per (slot, stencil cell)
                               (grids up to 1184 blocks; larger ones use 0); 4 = a
                               CTA per tile of cells walking the candidates staged
-                              in shared memory (DPD engines; mDPD runs 0); 5 = a
-                              thread per slot walking five column ranges of slots
-                              (cells z-1..z+1 of a column, contiguous under cell
-                              order 0 or 2; cell by cell where they are not)      */
+                              in shared memory (DPD engines; mDPD runs 0); 5 = five
+                              column ranges of slots per slot (cells z-1..z+1 of a
+                              column, contiguous under cell order 0 or 2; cell by
+                              cell where they are not), a thread per slot, or per
+                              (slot, range) on small grids under cell order 0     */
     int launch_mode;       /* 0 = small grids (up to 1184 blocks of 256 slots) run the
                               pair pass as one launch (schedule 4 in place of 8) and
                               the integrate as one, the step's bookkeeping in the
