@@ -1542,6 +1542,8 @@ int Engine::get_state(int rep, double* x, double* v, int* image, double* f)
         err = "corrupt tag in device state";
         return DPD_E_STATE;
     }
+    // 65536 values a thread and more: 24k particles stay with one thread (starting a second one can
+    // take longer than the copy), 384k take 16: 1010 us a state, 1225 with 131072 values a thread
     parallel_for(3 * n, [&](int64_t k0, int64_t k1) {
         if (x) memcpy(x + k0, o.x + k0, sizeof(double) * (k1 - k0));
         if (image) memcpy(image + k0, o.image + k0, sizeof(int) * (k1 - k0));
@@ -1549,7 +1551,7 @@ int Engine::get_state(int rep, double* x, double* v, int* image, double* f)
             for (int64_t k = k0; k < k1; k++) v[k] = o.v[k];
         if (f)
             for (int64_t k = k0; k < k1; k++) f[k] = o.f[k];
-    }, 131072);
+    }, 65536);
     if (spring)
         for (int64_t i = 0; i < n; i++) {
             const int t0 = R.sys.type[i] - 1;
