@@ -16,11 +16,11 @@ __global__ void k_aos_in(StepArgs a, const float* __restrict__ xin, const float*
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const RepDesc& d = a.reps[0];
     if (i == 0) {
-        RepState st = a.rstate[0];
+        // field by field: other threads of this launch raise bits of the status word
+        RepState& st = a.rstate[0];
         st.step = step;
         st.target = step;
         st.zero_pending = 1;
-        a.rstate[0] = st;
         if (force_build) a.build_flag[(*a.phase) & 1] = 1;
     }
     if (i >= n) return;
