@@ -1098,7 +1098,8 @@ int Engine::refresh_list()
 
 // Steps of a graph launch: 24000 particles take 32.1 us a step with 1, 29.2 with 8 (3000: 23.7
 // and 20.8; 192000: 71.9 and 70.4).  Making the graph of 8 takes 0.26 ms, what it saves in about
-// 120 steps, so an engine makes it for the run that takes it past DPD_GRAPH_AFTER steps.
+// 120 steps, so an engine makes it for the run that takes it past DPD_GRAPH_AFTER steps with its
+// present tuning.
 #define DPD_GRAPH_STEPS 8
 #define DPD_GRAPH_AFTER 120
 
@@ -1109,14 +1110,20 @@ int Engine::capture_steps(int n, cudaGraphExec_t* out)
         *out = nullptr;
     }
     cudaGraph_t g;
+    cudaGraphExec_t ge = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < n; k++) enqueue_step(stream_, nullptr, nullptr);
     cudaError_t e = cudaStreamEndCapture(stream_, &g);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
-    e = cudaGraphInstantiate(out, g, 0);
+    e = cudaGraphInstantiate(&ge, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
-    CK(cudaGraphUpload(*out, stream_));
+    e = cudaGraphUpload(ge, stream_);
+    if (e != cudaSuccess) {
+        cudaGraphExecDestroy(ge);
+        return cuda_fail(e, "cudaGraphUpload");
+    }
+    *out = ge;
     return DPD_OK;
 }
 
@@ -1128,6 +1135,7 @@ int Engine::build_graph()
         cudaGraphExecDestroy(graph_many_);
         graph_many_ = nullptr;
     }
+    graph_steps_ = 0;
     return e;
 }
 
@@ -1160,6 +1168,16 @@ int Engine::run_async(uint32_t nsteps)
     for (;;) {
         uint32_t end = last;
         for (auto& w : dumps_) end = std::min(end, next_dump(w.get(), s));
+        uint32_t left = end - s + 1;
+        // before anything of the run is launched, and a run without it goes on step by step: when
+        // it cannot be made (device memory is short, say) no state has moved and nothing is lost
+        if (!graph_many_ && left >= DPD_GRAPH_STEPS && graph_steps_ + left > DPD_GRAPH_AFTER) {
+            const std::string said = err;
+            if (capture_steps(DPD_GRAPH_STEPS, &graph_many_) != DPD_OK) {
+                err = said;
+                cudaGetLastError();
+            }
+        }
         if (ranks_dirty_) {
             const int e = upload_ranks();
             if (e) return e;
@@ -1172,11 +1190,7 @@ int Engine::run_async(uint32_t nsteps)
             enqueue_begin(stream_, end);
         }
         CK(cudaGetLastError());
-        uint32_t left = end - s + 1;
-        if (!graph_many_ && left >= DPD_GRAPH_STEPS && (uint64_t)s + left > DPD_GRAPH_AFTER) {
-            const int e = capture_steps(DPD_GRAPH_STEPS, &graph_many_);
-            if (e) return e;
-        }
+        graph_steps_ += left;
         for (; graph_many_ && left >= DPD_GRAPH_STEPS; left -= DPD_GRAPH_STEPS) CK(cudaGraphLaunch(graph_many_, stream_));
         for (; left > 0; left--) CK(cudaGraphLaunch(graph_, stream_));
         zero = false;
@@ -1278,7 +1292,7 @@ int Engine::time_steps(uint32_t nsteps, double* total_ms, double* pair_ms, int64
         if (e) return e;
         ranks_dirty_ = false;
     }
-    enqueue_begin(stream_, target);
+    // the graph before the drift: when it cannot be made, no state has moved
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     for (uint32_t k = 0; k < nsteps; k++) enqueue_step(stream_, ev[2 * k + 2], ev[2 * k + 3]);
@@ -1291,6 +1305,7 @@ int Engine::time_steps(uint32_t nsteps, double* total_ms, double* pair_ms, int64
     // upload the executable graph before the timed region (a first launch would otherwise
     // include the upload)
     CK(cudaGraphUpload(ge, stream_));
+    enqueue_begin(stream_, target);
     CK(cudaStreamSynchronize(stream_));
     CK(cudaEventRecord(ev[0], stream_));
     CK(cudaGraphLaunch(ge, stream_));

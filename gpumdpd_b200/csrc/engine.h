@@ -206,6 +206,7 @@ private:
     // within a step do; consecutive graph launches do not)
     cudaGraphExec_t graph_ = nullptr, graph_many_ = nullptr;
     int capture_steps(int n, cudaGraphExec_t* out);
+    uint64_t graph_steps_ = 0;  // steps run since the graphs of the present tuning were made
     int P_ = 0, C_ = 0, nmax_ = 16, maxb_ = 0;
     bool any_mdpd_ = false, any_dpd_ = false, bonds_ = false, rdf_ = false;
     bool any_spring_ = false, any_eos_ = false;  // some replica has a spring / an rvcm or recenter
