@@ -13,6 +13,7 @@
 
 #include "dump.h"
 #include "engine.h"
+#include "launch_rules.h"
 #include "kernels.cuh"
 #include "kernels_aos.cuh"
 #include "kernels_step.cuh"
@@ -796,18 +797,15 @@ static void pdl_launch_smem(void (*kern)(KArgs...), int grid, int block, size_t 
     cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-// the flattened schedules (4..9): one launch for any step (split = false) or two
+// the flattened schedules (4..9): one launch for any step (split = false) or two; alone: the
+// engine has the GPU to itself
 template <int STYLE, bool BONDS, bool FILT>
-static void launch_flat(bool split, cudaStream_t s, const StepArgs& a)
+static void launch_flat(bool split, bool alone, cudaStream_t s, const StepArgs& a)
 {
     const int threads = DPD_FLAT_WARPS * 32, grid = (a.P + threads - 1) / threads;
     if (!split) {
-        // several warps per 32 particles while the GPU has room for them: 24000 particles
-        // take 21.7 / 16.3 / 14.3 / 14.4 us with 1 / 2 / 4 / 8 parts, 81000 25.4 / 25.1 / 26.4
-        // with 1 / 2 / 4, 192000 44.2 / 44.3 / 50.0
-        const int warps = a.P / 32;
-        const int parts = warps <= 148 * 6 ? 4 : (warps <= 148 * 20 ? 2 : 1);
-        pdl_launch(k_pair_flat<STYLE, BONDS, FILT, FILT ? 12 : 16>, dim3(grid, parts), threads, s, a);
+        pdl_launch(k_pair_flat<STYLE, BONDS, FILT, FILT ? 12 : 16>, dim3(grid, flat_parts(a.P / 32, alone)), threads,
+                   s, a);
     } else {
         pdl_launch(k_pair_flat_split<STYLE, BONDS, FILT, FILT ? 16 : 20>, grid, threads, s, a);
         pdl_launch(k_pair_flat_logsteps<STYLE, BONDS, FILT>, std::min(grid, 148 * (FILT ? 12 : 16)), threads, s, a);
@@ -815,14 +813,14 @@ static void launch_flat(bool split, cudaStream_t s, const StepArgs& a)
 }
 
 template <int STYLE, bool BONDS>
-static void launch_pair2(int variant, bool filt, int grid, cudaStream_t s, const StepArgs& a)
+static void launch_pair2(int variant, bool filt, bool alone, int grid, cudaStream_t s, const StepArgs& a)
 {
     if (variant == 0) pdl_launch(k_pair<STYLE, BONDS>, grid, 256, s, a);
     else if (variant == 2) pdl_launch(k_pair_q<STYLE, BONDS, 4, true>, grid, 256, s, a);
     else if (variant == 3) pdl_launch(k_pair_q<STYLE, BONDS, 3, false>, grid, 256, s, a);
     else if (variant >= 4 && variant <= 9) {
-        if (filt) launch_flat<STYLE, BONDS, true>(variant >= 7, s, a);
-        else launch_flat<STYLE, BONDS, false>(variant >= 7, s, a);
+        if (filt) launch_flat<STYLE, BONDS, true>(variant >= 7, alone, s, a);
+        else launch_flat<STYLE, BONDS, false>(variant >= 7, alone, s, a);
     } else if (variant == 10) {
         pdl_launch(k_pair_entry<STYLE, BONDS>, (a.nmax * (a.P >> 5) + 7) / 8, 256, s, a);
     }
@@ -838,10 +836,10 @@ static void launch_pair2(int variant, bool filt, int grid, cudaStream_t s, const
 // entry (small grids); 11 (DPD engines): no list, the cell-tile kernel (kernels_tile.cuh)
 // after the counting sort
 template <int STYLE>
-static void launch_pair(int variant, bool bonds, bool filt, int grid, cudaStream_t s, const StepArgs& a)
+static void launch_pair(int variant, bool bonds, bool filt, bool alone, int grid, cudaStream_t s, const StepArgs& a)
 {
-    if (bonds) launch_pair2<STYLE, true>(variant, filt, grid, s, a);
-    else launch_pair2<STYLE, false>(variant, filt, grid, s, a);
+    if (bonds) launch_pair2<STYLE, true>(variant, filt, alone, grid, s, a);
+    else launch_pair2<STYLE, false>(variant, filt, alone, grid, s, a);
 }
 
 // Blocks of 256 slots up to which a thread per (slot, column group) builds the list: a step of
@@ -905,7 +903,8 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     // idle lanes cost more than the parallelism gains.  launch_mode 3 leaves them out: an
     // engine that shares the GPU with others (a server's cohorts) gains more from leaving
     // SMs to them than from spreading its own few pairs
-    const bool tiny = small && gp <= 148 && tune_.launch_mode != 3;
+    const bool alone = tune_.launch_mode != 3;
+    const bool tiny = small && gp <= 148 && alone;
     // schedule 11: no neighbour list, the cell-tile kernel after the counting sort
     const bool tile = use_tile();
     // a thread per list entry while its nmax warps per 32 slots fit the GPU at once (3000
@@ -917,7 +916,7 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     enqueue_build(s, !fused && !tile,
                   (tiny && (tune_.build_variant == 0 || tune_.build_variant == 5)) || tune_.build_variant == 3,
                   tune_.cell_order == 0,  // a run uploads the ranks of the tuning first
-                  small && tune_.launch_mode != 3 && gp <= DPD_SPREAD_BLOCKS);
+                  small && alone && gp <= DPD_SPREAD_BLOCKS);
     StepArgs sm = sa;  // mDPD: the force pass takes the density pass's list
     sm.nlist = b_.near_list;
     sm.ncount = b_.near_count;
@@ -946,9 +945,9 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
         else if (filt_) pdl_launch(k_build_pair<false, true, 12>, gw, threads, s, sa, ba);
         else pdl_launch(k_build_pair<false, false, 16>, gw, threads, s, sa, ba);
     } else if (any_dpd_) {
-        launch_pair<0>(variant, bonds_, filt_, gp, s, sa);
+        launch_pair<0>(variant, bonds_, filt_, alone, gp, s, sa);
     }
-    if (any_mdpd_) launch_pair<1>(variant, bonds_, false, gp, s, sm);
+    if (any_mdpd_) launch_pair<1>(variant, bonds_, false, alone, gp, s, sm);
     if (ev1) cudaEventRecordWithFlags(ev1, s, cudaEventRecordExternal);
     if (nang_ > 0) pdl_launch(k_angle, (nang_ + 255) / 256, 256, s, sa, angle_tbl_, angle_coef_, angle_wrep_, nang_);
     if (rdf_) pdl_launch(k_rdf, gp, 256, s, sa);
@@ -1986,10 +1985,10 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
     // the launch choices of enqueue_step for small and tiny grids: the list build with a thread
     // per (slot, stencil cell), the pair pass in one launch
     const bool small = tune_.launch_mode == 2 || ((tune_.launch_mode == 0 || tune_.launch_mode == 3) && gp <= 148 * 8);
-    const bool tiny = small && gp <= 148 && tune_.launch_mode != 3;
+    const bool alone = tune_.launch_mode != 3, tiny = small && gp <= 148 && alone;
     // a changed cell order waits for the next run: until then the device keeps the old ranks
     enqueue_build(stream_, true, (tiny && (tune_.build_variant == 0 || tune_.build_variant == 5)) || tune_.build_variant == 3,
-                  tune_.cell_order == 0 && !ranks_dirty_, small && tune_.launch_mode != 3 && gp <= DPD_SPREAD_BLOCKS);
+                  tune_.cell_order == 0 && !ranks_dirty_, small && alone && gp <= DPD_SPREAD_BLOCKS);
     StepArgs sm = sa;
     sm.nlist = b_.near_list;
     sm.ncount = b_.near_count;
@@ -2000,10 +1999,10 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
     if (pv == 8 && small) pv = 4;
     if (d.style == 0) {
         if (peratom) k_pair_peratom<0><<<gp, 256, 0, stream_>>>(sa, pe_slot_, vir_slot_);
-        else launch_pair<0>(pv, false, filt_, gp, stream_, sa);
+        else launch_pair<0>(pv, false, filt_, alone, gp, stream_, sa);
     } else {
         if (peratom) k_pair_peratom<1><<<gp, 256, 0, stream_>>>(sa, pe_slot_, vir_slot_);
-        else launch_pair<1>(pv, false, false, gp, stream_, sm);
+        else launch_pair<1>(pv, false, false, alone, gp, stream_, sm);
     }
     pdl_launch(k_aos_out, gp, 256, stream_, sa, d_force, d_pe, d_virial, pe_slot_, vir_slot_);
     CK(cudaGetLastError());

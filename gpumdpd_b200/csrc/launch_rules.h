@@ -1,0 +1,19 @@
+// launch_rules.h -- host rules that choose how a step's kernels are launched (plain C++).
+#pragma once
+
+namespace dpd {
+
+// Parts that the flattened pair schedule cuts the entries of 32 particles into, each a warp's
+// work, when it runs as one launch.  Several while the GPU has room for them: 24000 particles take
+// 21.7 / 16.3 / 14.3 / 14.4 us with 1 / 2 / 4 / 8 parts, 81000 25.4 / 25.1 / 26.4 with 1 / 2 / 4,
+// 192000 44.2 / 44.3 / 50.0.  An engine that shares the GPU with others (a server's cohorts) takes
+// one, since theirs fill the rest: 64 jobs at 64 jobs/s are served at 2.58 / 2.79 / 2.92 / 2.78 /
+// 2.82e9 particle-steps/s with one part and at 2.50 / 2.71 / 2.82 / 2.76 / 2.47e9 with parts by
+// size (five runs of each in turn).
+inline int flat_parts(int warps, bool alone)
+{
+    if (!alone) return 1;
+    return warps <= 148 * 6 ? 4 : (warps <= 148 * 20 ? 2 : 1);
+}
+
+}  // namespace dpd
