@@ -172,19 +172,17 @@ int Engine::layout()
         C_ += d.ncell + 1;
         d.tag_base = tag_base;
         tag_base += n;
-        const float cutf = (float)cut;
-        d.cut2 = cutf * cutf;
+        d.cut2 = cutoff2(cut);
         double rcm = 0, rdm = 0;
         for (auto& c : R.ff.coeff) {
             rcm = std::max(rcm, c[3]);
             rdm = std::max(rdm, c[4]);
         }
-        d.rcmax2 = (float)(rcm * rcm);
-        // not below the pairs' own rd^2, which are squared in float
-        d.rdmax2 = (float)rdm * (float)rdm;
+        d.rcmax2 = cutoff2(rcm);
+        d.rdmax2 = cutoff2(rdm);
         const float hs = (float)(R.in.skin * 0.5);
         d.hskin2 = hs * hs;
-        if (d.cut2 > d.rcmax2) filt_ = true;
+        if (lists_beyond(cut, rcm)) filt_ = true;
         d.skin_zero = R.in.skin == 0.0;
         d.ntypes = R.sys.n_atomtypes;
         d.coeff_off = coeff_off;
