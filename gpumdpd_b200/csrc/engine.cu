@@ -829,10 +829,10 @@ static void launch_pair2(int variant, bool filt, bool alone, int grid, cudaStrea
 // j-side forces by float4 reductions in L2, 4 blocks/SM; 2: warp pair-queue with the
 // i-side reduced through shared-memory atomics; 3: as 1 with 3 blocks/SM; 4, 5: flattened
 // warp schedule; 6: the flattened schedule with the list build fused into it (DPD; mDPD
-// falls back to 4); 7, 8 (the default) and 9: the flattened schedule as two launches,
-// non-log steps without FP64 sums at 40 warps/SM, log steps at 32; 10: one thread per list
-// entry (small grids); 11 (DPD engines): no list, the cell-tile kernel (kernels_tile.cuh)
-// after the counting sort
+// falls back to 4); 8 (the default; 7 and 9 are other names for it): the flattened schedule as
+// two launches, non-log steps without FP64 sums at 40 warps/SM, log steps at 32 (32 and 24 where
+// the list is filtered first); 10: one thread per list entry (small grids); 11 (DPD engines): no
+// list, the cell-tile kernel (kernels_tile.cuh) after the counting sort
 template <int STYLE>
 static void launch_pair(int variant, bool bonds, bool filt, bool alone, int grid, cudaStream_t s, const StepArgs& a)
 {
@@ -908,7 +908,7 @@ void Engine::enqueue_step(cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1)
     // a thread per list entry while its nmax warps per 32 slots fit the GPU at once (3000
     // particles, nmax 96: 8.3 us against 10.2 for the flattened schedule; 24000: 30.9 against 14.3)
     const bool entry = tiny && (int64_t)nmax_ * (P_ / 32) <= 148 * 64;
-    const int variant = tile ? 11 : (small && tune_.pair_variant == 8 ? (entry ? 10 : 4) : tune_.pair_variant);
+    const int variant = pair_schedule(tune_.pair_variant, tile, small, entry);
     // schedule 6: the DPD list build runs inside the pair kernel
     const bool fused = variant == 6 && !any_mdpd_;
     enqueue_build(s, !fused && !tile,
@@ -1993,8 +1993,7 @@ int Engine::pair_compute_aos(const float* d_pos, const float* d_vel, const int* 
     if (any_mdpd_) pdl_launch(k_density, (P_ + 32 * DPD_DENS_WARPS - 1) / (32 * DPD_DENS_WARPS), 32 * DPD_DENS_WARPS, stream_, sa, b_.near_list, b_.near_count);
     const bool peratom = d_pe || d_virial;
     // this entry builds the list itself: schedule 11 (no list) runs as the default 8
-    int pv = tune_.pair_variant == 11 ? 8 : tune_.pair_variant;
-    if (pv == 8 && small) pv = 4;
+    const int pv = pair_schedule(tune_.pair_variant, false, small, false);
     if (d.style == 0) {
         if (peratom) k_pair_peratom<0><<<gp, 256, 0, stream_>>>(sa, pe_slot_, vir_slot_);
         else launch_pair<0>(pv, false, filt_, alone, gp, stream_, sa);

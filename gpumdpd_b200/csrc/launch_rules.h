@@ -34,4 +34,15 @@ inline bool lists_beyond(double list_cut, double largest_rc)
     return cutoff2(list_cut) > cutoff2(largest_rc);
 }
 
+// The pair schedule that a step runs.  7, 8 and 9 are one schedule, the flattened one with log and
+// non-log steps split, and an engine that cannot run the cell tiles (11) takes it too; small grids
+// run it as one launch (4), or as a thread per list entry (10) where `entry` holds.
+inline int pair_schedule(int asked, bool tile, bool small, bool entry)
+{
+    if (tile) return 11;
+    const bool split = (asked >= 7 && asked <= 9) || asked == 11;
+    if (!split) return asked;
+    return small ? (entry ? 10 : 4) : 8;
+}
+
 }  // namespace dpd

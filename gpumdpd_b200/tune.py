@@ -14,7 +14,7 @@ src/force/pair_dpd.cu:613-616 eight threads per particle):
   above 0.  Only intervals that cannot miss a rebuild are tried: nl_f times the largest
   per-step displacement seen over a few steps, times 1.5, must stay below skin/2;
 - the pair schedule and its work split: a thread per particle (0), the warp pair queue
-  (1), the flattened warp schedule (4, 8, 9), and the cell-tile kernel without a list
+  (1), the flattened warp schedule (4, 8), and the cell-tile kernel without a list
   (11) with 1, 2 or 4 home cells per tile edge (or the engine's choice);
 - the launch mode (0: the fused small-grid launches where they apply; 1: never);
 - the cell order of the slots and the list build that goes with it: linear cells with the
@@ -31,8 +31,8 @@ import numpy as np
 from .engine import Batch, Engine
 
 SKINS = (0.0, 0.1, 0.2, 0.3)
-SCHEDULES = ({"pair_variant": 8}, {"pair_variant": 4}, {"pair_variant": 1}, {"pair_variant": 9},
-             {"pair_variant": 11, "tile": 0}, {"pair_variant": 11, "tile": 2}, {"pair_variant": 11, "tile": 4})
+SCHEDULES = ({"pair_variant": 8}, {"pair_variant": 4}, {"pair_variant": 1}, {"pair_variant": 11, "tile": 0},
+             {"pair_variant": 11, "tile": 2}, {"pair_variant": 11, "tile": 4})
 LAUNCH_MODES = (0, 1)
 INTERVALS = (1, 2, 5)
 LISTS = ({"cell_order": 0, "build_variant": 5}, {"cell_order": 1, "build_variant": 0})

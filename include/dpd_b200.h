@@ -88,7 +88,7 @@ typedef struct dpd_tuning {
                               4-5 = flattened warp schedule (small skins),
                               6 = flattened with the list build fused (DPD),
                               7-9 = flattened, log and non-log steps split (8 is
-                              the default; 7 and 9 run the same kernels),
+                              the default; 7 and 9 are other names for it),
                               10 = one thread per list entry, 11 = no neighbour
                               list: a CTA per tile of cells stages the tile's
                               neighbourhood in shared memory and evaluates its

@@ -11,6 +11,10 @@ WRAP = """
 #include "launch_rules.h"
 extern "C" int flat_parts(int warps, int alone) { return dpd::flat_parts(warps, alone != 0); }
 extern "C" int lists_beyond(double list_cut, double rc) { return dpd::lists_beyond(list_cut, rc); }
+extern "C" int pair_schedule(int asked, int tile, int small, int entry)
+{
+    return dpd::pair_schedule(asked, tile != 0, small != 0, entry != 0);
+}
 """
 
 
@@ -36,3 +40,20 @@ def test_a_list_cut_at_the_pair_cutoff_holds_nothing_beyond_it(rules):
         c = k / 100.0
         assert not rules.lists_beyond(c, c), c
         assert rules.lists_beyond(c + 0.01, c) and rules.lists_beyond(c, 0.99 * c)
+
+
+def test_names_of_one_schedule_are_launched_alike(rules):
+    for tile, small, entry in ((0, 0, 0), (0, 1, 0), (0, 1, 1)):
+        want = rules.pair_schedule(8, tile, small, entry)
+        assert want == (10 if entry else 4 if small else 8)
+        for other in (7, 9, 11):  # 11: an engine without the cell tiles
+            assert rules.pair_schedule(other, tile, small, entry) == want
+        for own in (0, 1, 2, 3, 4, 5, 6, 10):
+            assert rules.pair_schedule(own, tile, small, entry) == own
+    assert rules.pair_schedule(11, 1, 1, 0) == 11
+
+
+def test_the_tuner_times_a_schedule_once(rules):
+    from gpumdpd_b200 import tune
+    names = [(rules.pair_schedule(s["pair_variant"], s["pair_variant"] == 11, 0, 0), s.get("tile")) for s in tune.SCHEDULES]
+    assert len(set(names)) == len(names)
