@@ -43,38 +43,48 @@ def workload_name(args):
 
 def build_launches(system, skin, pair_variant=8):
     """Kernels of one list build: counting pass, scan (one launch when the cells fit one
-    4096-element block, else three), permutation (with the parity flip up to 1184 blocks
-    of 256 slots, else a separate flip), list (none with the cell-tile schedule 11)."""
+    4096-element block, two up to 1024 blocks, else three), permutation (with the parity flip
+    up to 1184 blocks of 256 slots, else a separate flip), list (none with the cell-tile
+    schedule 11)."""
     cells = int(np.prod(np.floor(system.box / (1.0 + skin)))) + 1
     slots = system.n + 31
-    return (2 if pair_variant == 11 else 3) + (1 if cells <= 4096 else 3) + \
+    return (2 if pair_variant == 11 else 3) + (1 if cells <= 4096 else 2 if cells <= 4096 * 1024 else 3) + \
         (0 if (slots + 255) // 256 <= 148 * 8 else 1)
 
 
+def list_capacity(system):
+    """Entries per slot of the engine's list: the reference's rule from the `neighbor` command,
+    in steps of 16 (src/force/neigh_list.cu:14-17)."""
+    t = next(ln.split() for ln in system.run_in.splitlines() if ln.startswith("neighbor"))
+    cut, rho = float(t[1]) + float(t[2]), float(t[3])
+    return (int(rho * 4.0 / 3.0 * math.pi * cut ** 3) + 16) // 16 * 16
+
+
 def pair_kernel_name(system, pair_variant):
-    """The pair kernel the engine launches for this system: on tiny grids (up to 148 blocks
-    of 256 slots) one thread per list entry, on small grids (up to 1184) the flattened
-    schedule as one launch, else the flattened schedule split by log steps."""
+    """The pair kernel the engine launches for this system: on tiny grids (up to 148 blocks of
+    256 slots) whose list entries the GPU's threads hold at once, one thread per list entry, on
+    small grids (up to 1184) the flattened schedule as one launch, else the flattened schedule
+    split by log steps."""
     gp = (system.n + 31 + 255) // 256
+    split = pair_variant in (7, 8, 9)
     if pair_variant == 11:
         return "k_tile + k_tile_logsteps (cell tiles staged in shared memory, no list)"
-    if pair_variant == 8 and gp <= 148:
+    if split and gp <= 148 and list_capacity(system) * ((system.n + 31) // 32) <= 148 * 64:
         return "k_pair_entry (thread per list entry, tiny grids)"
-    if pair_variant == 8 and gp <= 148 * 8:
+    if split and gp <= 148 * 8:
         return "k_pair_flat (flattened pair schedule, one launch on small grids)"
     return "k_pair_flat_split + k_pair_flat_logsteps (flattened pair schedule)"
 
 
 def step_launches(system, pair_variant):
-    """Kernels of one step after the list build: on small grids (up to 1184 blocks of 256
-    slots) the pair pass and the integrate with the bookkeeping are one launch each; else
-    the pair kernel(s), the integrate pair (non-log steps + log steps) and advance."""
+    """Kernels of one step after the list build: the many-body density pass, the pair kernel(s)
+    (two where log and non-log steps are split), and the integrate with the bookkeeping in one
+    launch on small grids (up to 1184 blocks of 256 slots), else the integrate pair (non-log
+    steps + log steps) and advance."""
     small = (system.n + 31 + 255) // 256 <= 148 * 8
-    if small and pair_variant == 8:
-        return 2
-    if pair_variant == 11:
-        return 2 + (1 if small else 3)
-    return (2 if pair_variant in (7, 8, 9) else 1) + 3
+    mdpd = any(ln.split()[:2] == ["pair_style", "mdpd"] for ln in system.run_in.splitlines())
+    two = (pair_variant == 11 and not mdpd) or (not small and pair_variant in (7, 8, 9, 11))
+    return int(mdpd) + (2 if two else 1) + (1 if small else 3)
 
 
 def thermo_every(args):
@@ -454,11 +464,11 @@ def run_ours(args, world, rank, local):
                      "pairs_per_step": pairs_per_step,
                      "saru_int_ops_per_pair": 130},
         "clocks": clk_summary,
-        # per step: the list-build kernels (counting pass, 1 or 3 scan launches, permutation,
+        # per step: the list-build kernels (counting pass, 1 to 3 scan launches, permutation,
         # list; each returns at once unless a build is flagged), the pair kernel(s), the
-        # integrate pair (non-log steps + log steps), advance; plus 2 before the graph
+        # integrate(s) and the bookkeeping; the drift before the first step is not timed
         "gpu_launches": int(args.steps * (build_launches(system, args.skin, pair_variant) +
-                                          step_launches(system, pair_variant)) + 2),
+                                          step_launches(system, pair_variant))),
         "impl": "ours",
     }
     if wipp and clk_summary.get("sm_mhz"):
