@@ -140,5 +140,5 @@ struct RepState {
 // Coefficient table entry per ordered type pair (3 float4):
 //  c0 = {A, gamma, sigma = sqrt(gamma)*sqrt(2kT)/sqrt(dt), 1/rc}: all that a DPD pair
 //       needs on a step without thermo
-//  c1 = {rc^2, 0.5*A*rc, B, 1/rd}
+//  c1 = {0, 0.5*A*rc, B, 1/rd}
 //  c2 = {rd^2, 0.25*B*rd, 15/(2 pi rd^3), rc}

@@ -359,13 +359,12 @@ int Engine::alloc_and_upload()
                 const auto& c = R.ff.coeff[tri_index(ti + 1, tj + 1, nt)];
                 const double A = c[0], B = c[1], gamma = c[2], rc = c[3], rd = c[4];
                 const size_t o = d.coeff_off + (size_t)(ti * nt + tj) * 3;
-                const float rcf = (float)rc;
                 coeff[o] = make_float4((float)A, (float)gamma, (float)(std::sqrt(gamma) * sig_scale), (float)(1.0 / rc));
-                coeff[o + 1] = make_float4(rcf * rcf, (float)(0.5 * A * rc), (float)B,
+                coeff[o + 1] = make_float4(0.0f, (float)(0.5 * A * rc), (float)B,
                                            rd > 0 ? (float)(1.0 / rd) : 0.0f);
                 const float rdf = (float)rd;
                 coeff[o + 2] = make_float4(rdf * rdf, (float)(0.25 * B * rd),
-                                           rd > 0 ? (float)(15.0 / (2.0 * M_PI * rd * rd * rd)) : 0.0f, rcf);
+                                           rd > 0 ? (float)(15.0 / (2.0 * M_PI * rd * rd * rd)) : 0.0f, (float)rc);
             }
         for (int t = 0; t < nt; t++) mass[d.mass_off + t] = make_float2((float)R.sys.masses[t], (float)(1.0 / R.sys.masses[t]));
         for (int b = 0; b < std::max(R.sys.n_bondtypes, 1); b++) {

@@ -370,6 +370,10 @@ __global__ void __launch_bounds__(F64_WARPS * 32, LOG ? 4 : 7) k64_force(F64Args
                     const int c0 = __shfl_sync(0xffffffffu, excl, c);
                     const int im = __shfl_sync(0xffffffffu, img, c);
                     if (q < nt) {
+                        // the box length is added to the neighbour before the difference is
+                        // taken, so across the boundary the two sides of a pair are negatives of
+                        // each other to the last bit of the coordinate, not exactly; the error
+                        // against the exact difference is the same
                         double4 rj = a.crec[(size_t)cc * a.cap + (t - c0)];
                         rj.x += (im & 3) == 1 ? 0.0 : ((im & 3) ? a.L[0] : -a.L[0]);
                         rj.y += ((im >> 2) & 3) == 1 ? 0.0 : (((im >> 2) & 3) ? a.L[1] : -a.L[1]);

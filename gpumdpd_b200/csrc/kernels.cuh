@@ -392,10 +392,12 @@ __device__ __forceinline__ void permute_slot(const BuildArgs& a, const int s)
 
 // The permutation.  FLIP (small grids, where a launch costs more than the work): the
 // last block to finish (a ticket counter) also flips the parity, counts the build of
-// every replica and resets the ticket.  Every block has read the parity before it takes
-// its ticket (nothing else of it is read by the last block, so no fence), and the list build
-// that follows waits for the whole grid.  Large grids leave the flip to k_flip: their tickets
-// take as long as that launch.
+// every replica and resets the ticket.  No fence, since the last block reads nothing that the
+// others write, and each read of the parity has been used (as the address of a load or store)
+// before its block's barrier, so before its ticket: the flip, which comes after every ticket,
+// cannot reach a read.  That holds only while no thread reads the parity for use after its
+// block's ticket.  The list build that follows waits for the whole grid.  Large grids leave the
+// flip to k_flip: their tickets take as long as that launch.
 template <bool FLIP>
 __global__ void k_permute(BuildArgs a, int nrep)
 {
@@ -404,7 +406,7 @@ __global__ void k_permute(BuildArgs a, int nrep)
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < a.P) permute_slot(a, s);
     if (!FLIP) return;
-    if (s < a.P) a.ncount[s] = 0;  // k_build_wide counts with atomics
+    if (s < a.P) a.ncount[s] = 0;  // k_build_wide and k_build_lin5 count with atomics
     __shared__ bool last;
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(a.ticket, 1u) == gridDim.x - 1u;

@@ -1691,7 +1691,11 @@ __global__ void k_advance(StepArgs a)
 
 // The step's bookkeeping of every replica by the last block of a launch (a ticket counter).
 // sums: the step has FP64 sums that the last block reads, so every block's are fenced before it
-// takes its ticket.  Otherwise the ticket only says that the block has read the step's state.
+// takes its ticket.  Otherwise the last block reads nothing that the others write, and there is no
+// fence: the step, phase and state words it then writes have been read and used by every block
+// before its barrier, so before its ticket, and a store that comes after every ticket cannot reach
+// those reads.  That holds only while no thread reads one of these words for use after its block's
+// ticket (but in the last block).
 __device__ __forceinline__ void advance_by_last_block(const StepArgs& a, const bool sums)
 {
     __shared__ bool last;

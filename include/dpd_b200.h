@@ -111,13 +111,20 @@ typedef struct dpd_tuning {
     int launch_mode;       /* 0 = small grids (up to 1184 blocks of 256 slots) run the
                               pair pass as one launch (schedule 4 in place of 8) and
                               the integrate as one, the step's bookkeeping in the
-                              integrate's last block; tiny ones (up to 148 blocks)
-                              also build the list with a thread per (slot, stencil
-                              cell) (in place of build variant 0 or 5) and run the pair
-                              pass with a thread per list entry (schedule 10);
-                              1 = never; 2 = always; 3 = as 0 without the tiny-grid
-                              kernels (the server's cohorts: engines that share
-                              the GPU run better on fewer, fuller blocks)         */
+                              integrate's last block, several warps sharing 32
+                              particles in the pair pass; up to 444 blocks build
+                              variant 5 under cell order 0 has a thread per (slot,
+                              column range).  Tiny grids (up to 148 blocks) build
+                              variant 0, and 5 under the other cell orders, with a
+                              thread per (slot, stencil cell), and run the pair pass
+                              with a thread per list entry (schedule 10) where their
+                              list entries fit the GPU's threads at once.
+                              1 = never; 2 = as 0, with the pair pass and the
+                              integrate in one launch each whatever the size;
+                              3 = as 0 without several threads per slot and without
+                              several warps per 32 particles (the server's cohorts:
+                              engines that share the GPU run better on fewer,
+                              fuller blocks)                                      */
     int tile;              /* pair_variant 11: home cells per tile edge, 1..6 (0 = the
                               engine's choice)                                    */
     int tile_capacity;     /* pair_variant 11: particles a CTA stages (0 = 1.5 times
