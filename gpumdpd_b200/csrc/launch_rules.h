@@ -7,9 +7,9 @@ namespace dpd {
 // work, when it runs as one launch.  Several while the GPU has room for them: 24000 particles take
 // 21.7 / 16.3 / 14.3 / 14.4 us with 1 / 2 / 4 / 8 parts, 81000 25.4 / 25.1 / 26.4 with 1 / 2 / 4,
 // 192000 44.2 / 44.3 / 50.0.  An engine that shares the GPU with others (a server's cohorts) takes
-// one, since theirs fill the rest: 64 jobs at 64 jobs/s are served at 2.58 / 2.79 / 2.92 / 2.78 /
-// 2.82e9 particle-steps/s with one part and at 2.50 / 2.71 / 2.82 / 2.76 / 2.47e9 with parts by
-// size (five runs of each in turn).
+// one, since theirs fill the rest: of ten pairs of runs taken in turn, a saturated stream of 64
+// jobs was served faster with one part in eight, by 5% on average (2.5e9 to 2.9e9
+// particle-steps/s; 2.4e9 to 2.8e9 with parts by size).
 inline int flat_parts(int warps, bool alone)
 {
     if (!alone) return 1;
