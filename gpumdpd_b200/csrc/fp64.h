@@ -39,6 +39,7 @@ public:
 private:
     int fail(cudaError_t e, const char* what);
     int upload_state(bool pos, bool vel);
+    int occupied_cells() const;
     int eval_forces(uint32_t step, bool log, bool binned, bool advance);
     int check_status();
     int log_row(uint32_t step);
@@ -59,6 +60,10 @@ private:
     int *img_ = nullptr, *type_ = nullptr, *cnt_ = nullptr, *ccode_ = nullptr;
     int* status_ = nullptr;
     int* cnt_next_ = nullptr;    // cell counts of the next binning
+    // sparse boxes: a warp per atom and steps of separate kernels, without the buffers of fused steps
+    // (xn_, vn_, craw_); each atom's cell where it came first, else -1, of this and the last binning
+    bool sparse_ = false;
+    int *owner_ = nullptr, *owner_prev_ = nullptr;
     int* craw_ = nullptr;        // atom indices appended to each cell, cap_ per cell
     double4* crec_ = nullptr;    // cell records in index order (position, atom index), cap_ per cell
     int *bstart_ = nullptr, *astart_ = nullptr;

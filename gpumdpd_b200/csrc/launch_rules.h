@@ -45,4 +45,16 @@ inline int pair_schedule(int asked, bool tile, bool small, bool entry)
     return small ? (entry ? 10 : 4) : 8;
 }
 
+// Whether the FP64 engine takes its forces with a warp per atom (steps of five kernels) rather than a
+// warp per cell (steps of two).  In units of 0.2 ns a step, fitted to runs of 1000 to 300000 atoms at
+// densities of 0.02 to 2: an occupied cell takes 10 and an empty one 1, since 4144 warps run at a time
+// and each is a chain of loads; an atom takes 4 and its neighbours 1 for each atom of a cell; the
+// longer step 62000 more.  us a step with a warp per atom and per cell, 100000 atoms: density 0.05
+// 83 / 488, 0.5 95 / 207, 1.0 106 / 139, 1.5 120 / 117, 2.0 123 / 100; 10000 atoms: 0.05 25 / 55, 0.5
+// 27 / 27, 1.0 29 / 22; 1000 atoms at 0.05 19 / 12.
+inline bool atom_pass(double n, double ncell, double occupied)
+{
+    return 10.0 * occupied + ncell > 62000.0 + 4.0 * n + n * (n / ncell);
+}
+
 }  // namespace dpd
