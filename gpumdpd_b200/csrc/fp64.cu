@@ -1015,7 +1015,10 @@ int EngineF64::init(Replica&& rep)
     F64_CK(dalloc64(&cnt_, (size_t)ncell_, bytes_));
     F64_CK(dalloc64(&cnt_next_, (size_t)ncell_, bytes_));
     // the occupied cells are counted where they can matter: min(n, ncell) is the most there can be
-    sparse_ = atom_pass(n_, ncell_, std::min(n_, ncell_)) && atom_pass(n_, ncell_, occupied_cells());
+    const int most = std::min(n_, ncell_);
+    const int occupied = atom_pass(n_, ncell_, most) || atom_pass_logged(n_, most) ? occupied_cells() : most;
+    sparse_ = atom_pass(n_, ncell_, occupied);
+    log_by_atom_ = sparse_ || atom_pass_logged(n_, occupied);
     if (sparse_) {
         F64_CK(dalloc64(&owner_, n, bytes_));
         F64_CK(dalloc64(&owner_prev_, n, bytes_));
@@ -1144,12 +1147,10 @@ int EngineF64::eval_forces(uint32_t step, bool log, bool binned, bool advance)
     else launch_dep(k64_sort_cells, (int)(((size_t)ncell_ * 8 + 255) / 256), 256, 0, stream_, a, ncell_);
     if (a.style == 1) launch_dep(k64_density, gw, 256, 0, stream_, a);
     const int gf = (ncell_ + F64_WARPS - 1) / F64_WARPS, tf = F64_WARPS * 32;  // a warp per cell
-    if (sparse_) {
-        const int ga = (n_ + F64_ATOM_WARPS - 1) / F64_ATOM_WARPS, ta = F64_ATOM_WARPS * 32;
-        if (log) launch_dep(k64_force_atom<true>, ga, ta, 0, stream_, a, step);
-        else launch_dep(k64_force_atom<false>, ga, ta, 0, stream_, a, step);
-        std::swap(owner_, owner_prev_);
-    } else if (log) launch_dep(k64_force<true, false>, gf, tf, F64_WARPS * sizeof(F64Warp<true>), stream_, a, step, ncell_);
+    const int ga = (n_ + F64_ATOM_WARPS - 1) / F64_ATOM_WARPS, ta = F64_ATOM_WARPS * 32;  // a warp per atom
+    if (log && log_by_atom_) launch_dep(k64_force_atom<true>, ga, ta, 0, stream_, a, step);
+    else if (sparse_) launch_dep(k64_force_atom<false>, ga, ta, 0, stream_, a, step);
+    else if (log) launch_dep(k64_force<true, false>, gf, tf, F64_WARPS * sizeof(F64Warp<true>), stream_, a, step, ncell_);
     else if (!advance)
         launch_dep(k64_force<false, false>, gf, tf, F64_WARPS * sizeof(F64Warp<false>), stream_, a, step, ncell_);
     else {
@@ -1159,6 +1160,7 @@ int EngineF64::eval_forces(uint32_t step, bool log, bool binned, bool advance)
     }
     // the sort has cleared the other counts: the next binning fills them
     std::swap(cnt_, cnt_next_);
+    std::swap(owner_, owner_prev_);
     F64_CK(cudaGetLastError());
     return DPD_OK;
 }

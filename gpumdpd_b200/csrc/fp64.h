@@ -63,6 +63,7 @@ private:
     // sparse boxes: a warp per atom and steps of separate kernels, without the buffers of fused steps
     // (xn_, vn_, craw_); each atom's cell where it came first, else -1, of this and the last binning
     bool sparse_ = false;
+    bool log_by_atom_ = false;  // logged steps take the forces with a warp per atom
     int *owner_ = nullptr, *owner_prev_ = nullptr;
     int* craw_ = nullptr;        // atom indices appended to each cell, cap_ per cell
     double4* crec_ = nullptr;    // cell records in index order (position, atom index), cap_ per cell

@@ -12,6 +12,7 @@ WRAP = """
 extern "C" int flat_parts(int warps, int alone) { return dpd::flat_parts(warps, alone != 0); }
 extern "C" int lists_beyond(double list_cut, double rc) { return dpd::lists_beyond(list_cut, rc); }
 extern "C" int atom_pass(double n, double ncell, double occupied) { return dpd::atom_pass(n, ncell, occupied); }
+extern "C" int atom_pass_logged(double n, double occupied) { return dpd::atom_pass_logged(n, occupied); }
 extern "C" int pair_schedule(int asked, int tile, int small, int entry)
 {
     return dpd::pair_schedule(asked, tile != 0, small != 0, entry != 0);
@@ -27,6 +28,7 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-o", so, str(d / "wrap.cpp")], check=True)
     lib = ctypes.CDLL(so)
     lib.atom_pass.argtypes = [ctypes.c_double] * 3
+    lib.atom_pass_logged.argtypes = [ctypes.c_double] * 2
     lib.lists_beyond.argtypes = [ctypes.c_double, ctypes.c_double]
     return lib
 
@@ -84,3 +86,10 @@ def test_fp64_pass_of_atoms_that_stay_together(rules):
     # warp per cell, 109 with a warp per atom
     for ncell in (12000, 48000, 96000):
         assert not rules.atom_pass(24000, ncell, 4000)
+
+
+@pytest.mark.parametrize("n,rho,by_atom", [(10000, 0.5, 1), (20000, 1.0, 1), (100000, 1.5, 1), (100000, 2.0, 0),
+                                           (3000, 3.0, 0), (3000000, 3.0, 0)])
+def test_fp64_pass_of_logged_steps(rules, n, rho, by_atom):
+    import math
+    assert rules.atom_pass_logged(n, n / rho * (1.0 - math.exp(-rho))) == by_atom
