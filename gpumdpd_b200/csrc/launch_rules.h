@@ -4,15 +4,20 @@
 namespace dpd {
 
 // Parts that the flattened pair schedule cuts the entries of 32 particles into, each a warp's
-// work, when it runs as one launch.  Several while the GPU has room for them: 24000 particles take
-// 21.7 / 16.3 / 14.3 / 14.4 us with 1 / 2 / 4 / 8 parts, 81000 25.4 / 25.1 / 26.4 with 1 / 2 / 4,
-// 192000 44.2 / 44.3 / 50.0.  An engine that shares the GPU with others (a server's cohorts) takes
-// one, since theirs fill the rest: of ten pairs of runs taken in turn, a saturated stream of 64
-// jobs was served faster with one part in eight, by 5% on average (2.5e9 to 2.9e9
-// particle-steps/s; 2.4e9 to 2.8e9 with parts by size).
+// work, when it runs as one launch.  Several while the GPU has room for them (us a step or of the
+// pass with 1 / 2 / 4 / 8 / 16 / 32 parts, "-" not measured): 2000 particles at density 10, skin 0.3
+// - / 33 / 24 / 19 / 17 / 16; 4000 at 3 - / 19 / 17 / 16 / 15 / 17, at 25 - / 64 / 41 / 30 / 24 / 25;
+// 8000 at 3 - / 19 / 17 / 16 / 18 / 21, at 25 - / 64 / 43 / 32 / 32 / 31; 16000 at 3 - / 20 / 18 / 19 /
+// 21 / 27; the pass at 24000 22 / 16.3 / 14.3 / 14.4, at 81000 25.4 / 25.1 / 26.4, at 192000 44.2 /
+// 44.3 / 50.  An engine that shares the GPU with others (a server's cohorts) takes one, since theirs
+// fill the rest: of ten pairs of runs taken in turn, a saturated stream of 64 jobs was served faster
+// with one part in eight, by 5% on average (2.5e9 to 2.9e9 particle-steps/s; 2.4e9 to 2.8e9 with 4
+// and 2 by size).
 inline int flat_parts(int warps, bool alone)
 {
     if (!alone) return 1;
+    if (warps <= 148) return 16;
+    if (warps <= 148 * 2) return 8;
     return warps <= 148 * 6 ? 4 : (warps <= 148 * 20 ? 2 : 1);
 }
 

@@ -34,9 +34,10 @@ def rules(tmp_path_factory):
 
 
 def test_engines_that_share_the_gpu_take_one_warp_per_32_particles(rules):
-    for warps in (1, 94, 148 * 6, 148 * 6 + 1, 148 * 20, 148 * 20 + 1, 9472):
+    for warps, alone in ((1, 16), (148, 16), (149, 8), (296, 8), (297, 4), (148 * 6, 4), (148 * 6 + 1, 2),
+                         (148 * 20, 2), (148 * 20 + 1, 1), (9472, 1)):
         assert rules.flat_parts(warps, 0) == 1
-        assert rules.flat_parts(warps, 1) == (4 if warps <= 148 * 6 else 2 if warps <= 148 * 20 else 1)
+        assert rules.flat_parts(warps, 1) == alone
 
 
 def test_a_list_cut_at_the_pair_cutoff_holds_nothing_beyond_it(rules):
