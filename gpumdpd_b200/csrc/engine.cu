@@ -126,6 +126,50 @@ int Engine::upload_ranks()
     return DPD_OK;
 }
 
+#define DPD_SMALL_BLOCKS (148 * 8)  // blocks of 256 slots up to which a grid is small
+
+// Mean entries of a particle's half list by the mean density, or (local) by the density of the cells
+// that particles are in: those of 128 of them, evenly taken from the input, whose particles one pass
+// over all positions counts
+static double mean_half_list(const Replica& R, bool local)
+{
+    const RepDesc& d = R.desc;
+    const double cut = R.in.global_cut + R.in.skin, sphere = 2.0 / 3.0 * M_PI * cut * cut * cut;
+    const double cell = R.box_len[0] * R.box_len[1] * R.box_len[2] / d.ncell;
+    if (!local) return sphere * d.n_real / (cell * d.ncell);
+    auto cell_of = [&](int64_t i) {
+        int c = 0;
+        for (int k = 0; k < 3; k++) {
+            double q = (R.sys.x[3 * i + k] - d.lo[k]) / R.box_len[k];
+            if (!std::isfinite(q)) q = 0.0;  // an error later
+            q -= std::floor(q);
+            c = c * d.nc[k] + std::min((int)(q * d.nc[k]), d.nc[k] - 1);
+        }
+        return c;
+    };
+    const int ns = std::min(d.n_real, 128);
+    std::vector<int> at(ns);
+    std::vector<char> mark(65536, 0);  // most cells are told apart by their low bits
+    for (int k = 0; k < ns; k++) {
+        at[k] = cell_of((int64_t)k * d.n_real / ns);
+        mark[at[k] & 65535] = 1;
+    }
+    std::sort(at.begin(), at.end());
+    std::vector<std::atomic<int>> held(ns);  // by the first of equal cells
+    for (auto& h : held) h = 0;
+    parallel_for(d.n_real, [&](int64_t i0, int64_t i1) {
+        for (int64_t i = i0; i < i1; i++) {
+            const int c = cell_of(i);
+            if (!mark[c & 65535]) continue;
+            const auto it = std::lower_bound(at.begin(), at.end(), c);
+            if (it != at.end() && *it == c) held[it - at.begin()]++;
+        }
+    });
+    double others = 0;  // particles beside the sampled one in its cell
+    for (int k = 0; k < ns; k++) others += held[std::lower_bound(at.begin(), at.end(), at[k]) - at.begin()] - 1;
+    return sphere * others / ns / cell;
+}
+
 int Engine::layout()
 {
     P_ = 0;
@@ -134,6 +178,7 @@ int Engine::layout()
     maxb_ = 0;
     int tag_base = 0, coeff_off = 0, mass_off = 0, bond_off = 0, rdf_off = 0;
     any_mdpd_ = any_dpd_ = bonds_ = rdf_ = any_gc_ = filt_ = false;
+    std::vector<char> beyond(reps_.size());
     for (size_t r = 0; r < reps_.size(); r++) {
         Replica& R = reps_[r];
         RepDesc& d = R.desc;
@@ -182,7 +227,8 @@ int Engine::layout()
         d.rdmax2 = cutoff2(rdm);
         const float hs = (float)(R.in.skin * 0.5);
         d.hskin2 = hs * hs;
-        if (lists_beyond(cut, rcm)) filt_ = true;
+        beyond[r] = lists_beyond(cut, rcm) && R.ff.pair_style == 0;
+        if (beyond[r]) filt_ = true;
         d.skin_zero = R.in.skin == 0.0;
         d.ntypes = R.sys.n_atomtypes;
         d.coeff_off = coeff_off;
@@ -231,6 +277,11 @@ int Engine::layout()
             maxb_ = std::max(maxb_, R.maxb);
         }
         rank_cells(R);
+    }
+    if (filt_ && (P_ + 255) / 256 > DPD_SMALL_BLOCKS) {
+        filt_ = false;
+        for (size_t r = 0; r < reps_.size() && !filt_; r++)
+            filt_ = beyond[r] && (filter_pays(mean_half_list(reps_[r], false)) || filter_pays(mean_half_list(reps_[r], true)));
     }
     if (maxb_ > 16) {
         err = "an atom has more than 16 bonds";

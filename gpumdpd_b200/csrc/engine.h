@@ -211,7 +211,7 @@ private:
     bool any_mdpd_ = false, any_dpd_ = false, bonds_ = false, rdf_ = false;
     bool any_spring_ = false, any_eos_ = false;  // some replica has a spring / an rvcm or recenter
     bool any_gc_ = false;                         // some replica has a temp/rho/msd/tf/wall_contact compute
-    bool filt_ = false;                           // some replica lists entries beyond its largest pair cutoff
+    bool filt_ = false;                           // the flattened pair pass filters its lists first
     bool any_motion_ = false, any_twowall_ = false, any_wallc_ = false;  // fix move/wall_reflect, two_wall, wall_contact
     // the integrate variant with group fixes and computes
     bool ext() const { return any_spring_ || any_eos_ || any_gc_ || any_motion_ || any_twowall_; }

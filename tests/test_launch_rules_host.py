@@ -13,6 +13,7 @@ extern "C" int flat_parts(int warps, int alone) { return dpd::flat_parts(warps, 
 extern "C" int lists_beyond(double list_cut, double rc) { return dpd::lists_beyond(list_cut, rc); }
 extern "C" int atom_pass(double n, double ncell, double occupied) { return dpd::atom_pass(n, ncell, occupied); }
 extern "C" int atom_pass_logged(double n, double occupied) { return dpd::atom_pass_logged(n, occupied); }
+extern "C" int filter_pays(double half_list) { return dpd::filter_pays(half_list); }
 extern "C" int pair_schedule(int asked, int tile, int small, int entry)
 {
     return dpd::pair_schedule(asked, tile != 0, small != 0, entry != 0);
@@ -29,6 +30,7 @@ def rules(tmp_path_factory):
     lib = ctypes.CDLL(so)
     lib.atom_pass.argtypes = [ctypes.c_double] * 3
     lib.atom_pass_logged.argtypes = [ctypes.c_double] * 2
+    lib.filter_pays.argtypes = [ctypes.c_double]
     lib.lists_beyond.argtypes = [ctypes.c_double, ctypes.c_double]
     return lib
 
@@ -94,3 +96,10 @@ def test_fp64_pass_of_atoms_that_stay_together(rules):
 def test_fp64_pass_of_logged_steps(rules, n, rho, by_atom):
     import math
     assert rules.atom_pass_logged(n, n / rho * (1.0 - math.exp(-rho))) == by_atom
+
+
+@pytest.mark.parametrize("rho,skin,pays", [(0.1, 0.3, 0), (0.3, 0.3, 0), (0.1, 1.0, 0), (0.2, 1.0, 1), (1.0, 0.3, 1),
+                                           (3.0, 0.3, 1)])
+def test_lists_of_dilute_systems_are_not_filtered(rules, rho, skin, pays):
+    import math
+    assert rules.filter_pays(rho * 2.0 / 3.0 * math.pi * (1.0 + skin) ** 3) == pays
