@@ -10,9 +10,9 @@ namespace dpd {
 // 8000 at 3 - / 19 / 17 / 16 / 18 / 21, at 25 - / 64 / 43 / 32 / 32 / 31; 16000 at 3 - / 20 / 18 / 19 /
 // 21 / 27; the pass at 24000 22 / 16.3 / 14.3 / 14.4, at 81000 25.4 / 25.1 / 26.4, at 192000 44.2 /
 // 44.3 / 50.  An engine that shares the GPU with others (a server's cohorts) takes one, since theirs
-// fill the rest: of ten pairs of runs taken in turn, a saturated stream of 64 jobs was served faster
-// with one part in eight, by 5% on average (2.5e9 to 2.9e9 particle-steps/s; 2.4e9 to 2.8e9 with 4
-// and 2 by size).
+// fill the rest: of 22 pairs of runs taken in turn, a saturated stream of 64 jobs was served faster
+// with one part in 14, by 2.5% on average (2.1e9 to 2.9e9 particle-steps/s either way, as the host's
+// load allows).
 inline int flat_parts(int warps, bool alone)
 {
     if (!alone) return 1;
